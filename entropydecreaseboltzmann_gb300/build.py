@@ -25,6 +25,7 @@ COMMON = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler",
 UNITS = {
     "edb_capi.cu": [],
     "edb_kernels_calq.cu": [],
+    "edb_kernels_calqtc.cu": [],
     "edb_kernels_calq64x.cu": [],
     "edb_kernels_calq64f.cu": [],
     "edb_kernels_conserve.cu": [],

@@ -136,6 +136,7 @@ struct edb_qcalc {
 
 // Grows the qcalc's solve-pair buffer to hold S solves (not under capture).
 static edb_status qcalc_pairs(edb_qcalc *q, int S) {
+  if (tc_takes(q->d.N)) return EDB_OK;  // no pair layout there
   const size_t need = calq32_pair_bytes(q->d.N, S);
   if (need <= q->pairs_bytes) return EDB_OK;
   EDB_CUDA(cudaDeviceSynchronize());
@@ -561,6 +562,11 @@ extern "C" edb_status edb_qcalc_calQ_batch_f32_device(edb_qcalc *q, int S, const
 static edb_status autotune_c32(edb_qcalc *q, int S, const float2 *d_fin, float2 *d_Qout,
                                cudaStream_t st, int C, float4 *d_partial, float4 *d_pairs,
                                int *chosen, int persist = -1) {
+  if (tc_takes(q->d.N)) {  // one shape, nothing to time
+    (C > 1 ? q->c32_variant_split : q->c32_variant)[s_bucket(S)] = 0;
+    if (chosen) *chosen = 0;
+    return EDB_OK;
+  }
   cudaEvent_t e0, e1;
   EDB_CUDA(cudaEventCreate(&e0));
   EDB_CUDA(cudaEventCreate(&e1));
@@ -1298,7 +1304,8 @@ extern "C" edb_status edb_batch_create(edb_qcalc *q, const edb_batch_desc *d, ed
   for (int i = 0; i < nstage && rc == EDB_OK; ++i) rc = dalloc(&b->Fs[i], n);
   for (int i = 0; i < nq && rc == EDB_OK; ++i) rc = dalloc(&b->Qs[i], n);
   if (rc == EDB_OK) rc = dalloc(&b->in32, n);
-  if (rc == EDB_OK) rc = dalloc(&b->pairs, calq32_pair_bytes(d->N, d->S) / sizeof(float4));
+  if (rc == EDB_OK && !tc_takes(d->N))
+    rc = dalloc(&b->pairs, calq32_pair_bytes(d->N, d->S) / sizeof(float4));
   if (rc == EDB_OK) rc = dalloc(&b->state, (size_t)d->S);
   if (rc == EDB_OK) rc = dalloc(&b->state_init, (size_t)d->S);
   if (rc == EDB_OK) {

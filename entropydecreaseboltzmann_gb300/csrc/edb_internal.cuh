@@ -158,10 +158,36 @@ __host__ __device__ inline int c32_plane_pos(int N, int k1, int l1) {
   if (l1 > k1 && l1 <= (k1 + N) / 2) return k1 / 2 + 1 + (l1 - k1 - 1);
   return -1;
 }
+// The tensor-core form of the batched kernel (edb_kernels_calqtc.cu) takes the
+// sizes from 13 to 32 whose lines are no multiple of 16 bytes (N % 4 != 0): its
+// operands are staged by plain loads of any width, where calq32_kernel falls
+// back to its plain-load path.  Measured against that path, S = 1, 256 and 4096
+// (S = 256 where 4096 is missing): N = 13 4.8x, 1.33x, 1.11x; N = 17 4.9x, 1.64x,
+// 1.50x; N = 23 5.7x, 2.6x; N = 31 6.9x, 4.0x.  Below 13 a step's tile is mostly
+// empty (N = 11: 4.6x at S = 1 but 0.79x at 4096); at N % 4 == 0 calq32_kernel's
+// tensor-copy path is faster at all but a few solves (512 x N = 24: 10.5 ms against
+// 15.6); and one size uses one kernel whatever S is, so that a solve's bits do not
+// depend on its batch.  Above 32 a line no longer fits the lanes and columns.
+inline bool tc_takes(int N) { return N >= 13 && N <= 32 && N % 4 != 0; }
+// CL l3 values per step, V steps per (l1, m2) line pair, NC weight columns,
+// staged-plane row pitch.
+struct TcGeom {
+  int CL, V, NC, pitch;
+};
+TcGeom tc_geom(int N);
 inline long long c32_table_floats(int N) {
+  if (tc_takes(N)) {
+    const TcGeom g = tc_geom(N);
+    return (long long)N * c32_maxlist(N) * N * g.V * 128 * g.NC;
+  }
   const long long NQ = (long long)N * N * N;
   return (long long)N * c32_maxlist(N) * N * NQ;
 }
+// Results in Q (C == 1) or, per chunk, in partial (calq32_reduce_kernel's form).
+edb_status launch_calqtc(int N, int S, const float *d_B32, const float2 *d_fin, float2 *d_Q, int C,
+                         float4 *d_partial, cudaStream_t st);
+// The batched kernels' status word on the current device.
+edb_status calq32_status_ptr(int **p);
 // variant in [0, calq32_variants()) selects the solve group and CTA shape
 // (see the kernel).  C > 1 splits the l1 planes into C chunks reduced in
 // order in FP64; d_partial then holds C * S * N^3 float4.  Pair variants

@@ -183,8 +183,9 @@ edb_status launch_calq64_reduce(const QParams &p, int nchunk, const double2 *d_p
 // inside an l1-plane.  All waits are bounded: a wait that runs out marks the
 // thread, the block leaves together at the next block barrier
 // (__syncthreads_or), drains its copies and sets a device status word.
-// Widths that are not multiples of 16 bytes or below 8 (N % 4 != 0, N < 8)
-// take the same compute path with cooperative plain loads instead of TMA.
+// Widths below 8, inputs that are not 16-byte aligned, and N % 4 != 0 outside
+// 13..32 take the same compute path with cooperative plain loads instead of TMA
+// (N % 4 != 0 inside: edb_kernels_calqtc.cu).
 //
 // Arithmetic, per term and solve, in three packed f32x2 instructions that carry
 // the six FP32 operations of the term:
@@ -1491,12 +1492,25 @@ static edb_status c32_setup(int N, int S, const C32Variant &vr, int C, const flo
   return EDB_OK;
 }
 
+static edb_status launch_c32_reduce(int N, int S, int C, const float4 *d_partial, float2 *d_Q,
+                                    cudaStream_t st) {
+  const long long n = (long long)S * N * N * N;
+  const long long blocks = std::min<long long>((n + 255) / 256, 16LL * device_sm_count());
+  calq32_reduce_kernel<<<(unsigned)blocks, 256, 0, st>>>(n, C, d_partial, d_Q);
+  EDB_LAUNCHED();
+  return EDB_OK;
+}
+
 edb_status launch_calq32_batch(int N, int S, const float *d_B32, const float2 *d_fin, float2 *d_Q,
                                cudaStream_t st, int variant, int C, float4 *d_partial,
                                float4 *d_pairs, int persist) {
   if (variant < 0 || variant >= calq32_variants()) variant = 0;
   if (C < 1 || C > N) return fail(EDB_EINVAL, "calq32: chunk count must be in [1, N]");
   if (C > 1 && !d_partial) return fail(EDB_EINVAL, "calq32: chunks need a partial-sum buffer");
+  if (tc_takes(N)) {  // one shape: every variant is the same launch
+    EDB_TRY(launch_calqtc(N, S, d_B32, d_fin, d_Q, C, d_partial, st));
+    return C == 1 ? EDB_OK : launch_c32_reduce(N, S, C, d_partial, d_Q, st);
+  }
   const C32Variant &vr = kC32Variants[variant];
   if (vr.pair && !d_pairs) return fail(EDB_EINVAL, "calq32: pair variants need a pair buffer");
   const int SG = SC * vr.ws;
@@ -1514,11 +1528,7 @@ edb_status launch_calq32_batch(int N, int S, const float *d_B32, const float2 *d
     one.partial = d_partial;
     EDB_TRY(launch_calq32_multi(1, &one, variant, st, persist < 0));
     if (C == 1) return EDB_OK;
-    const long long n = (long long)S * N * N * N;
-    const long long blocks = std::min<long long>((n + 255) / 256, 16LL * device_sm_count());
-    calq32_reduce_kernel<<<(unsigned)blocks, 256, 0, st>>>(n, C, d_partial, d_Q);
-    EDB_LAUNCHED();
-    return EDB_OK;
+    return launch_c32_reduce(N, S, C, d_partial, d_Q, st);
   }
   dim3 grid((unsigned)(((S + SG - 1) / SG) * C), (unsigned)N, (unsigned)su.tiles);
   if (vr.pair) {
@@ -1534,11 +1544,7 @@ edb_status launch_calq32_batch(int N, int S, const float *d_B32, const float2 *d
                                          su.NST, su.NPL, C, su.GB, d_B32, src, d_Q, d_partial,
                                          su.maps, st);
   if (rc != EDB_OK || C == 1) return rc;
-  const long long n = (long long)S * N * N * N;
-  const long long blocks = std::min<long long>((n + 255) / 256, 16LL * device_sm_count());
-  calq32_reduce_kernel<<<(unsigned)blocks, 256, 0, st>>>(n, C, d_partial, d_Q);
-  EDB_LAUNCHED();
-  return EDB_OK;
+  return launch_c32_reduce(N, S, C, d_partial, d_Q, st);
 }
 
 template <int V>
@@ -1655,6 +1661,11 @@ edb_status launch_calq32_multi(int ntab, const C32MultiIn *in, int variant, cuda
   const cudaError_t fe = queue ? cudaFreeAsync(mt.queue, st) : cudaSuccess;
   if (rc != EDB_OK) return rc;
   if (fe != cudaSuccess) return cuda_fail(fe, "cudaFreeAsync(calq32 multi queue)");
+  return EDB_OK;
+}
+
+edb_status calq32_status_ptr(int **p) {
+  EDB_CUDA(cudaGetSymbolAddress(reinterpret_cast<void **>(p), g_calq32_status));
   return EDB_OK;
 }
 

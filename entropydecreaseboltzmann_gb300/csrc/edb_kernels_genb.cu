@@ -12,6 +12,8 @@
 // -fmad=false: products and sums are rounded in the reference's order.
 #include <math.h>
 
+#include <algorithm>
+
 #include "edb_internal.cuh"
 
 namespace edb {
@@ -278,6 +280,58 @@ __global__ void genB_kernel(int N, int filter, double rval, const double *__rest
   }
 }
 
+// The pair table of the tensor-core batched kernel (tc_takes), the entries of
+// genB_kernel's in the order that kernel reads: one step's weights are 128 lanes
+// x NC columns, [k1][p][m2][v][j / 4][lane][j % 4].  Lane k2 CL + c, column j
+// of (k1, p, m2, v) weights the pair l = (l1 of p, k2 - m2, v CL + c),
+// m = (k1 - l1, m2, j - v CL), all mod N; places without a pair are zero.  One
+// thread writes the four columns of a 16-byte word.
+__global__ void genB32_tc_kernel(int N, int filter, double rval, const double *__restrict__ T,
+                                 int amax, const double *__restrict__ sigma,
+                                 const double *__restrict__ Bmm, TcGeom g, long long words,
+                                 float4 *__restrict__ out) {
+  const int n = (N - 1) / 2, Q4 = g.NC / 4, ML = c32_maxlist(N);
+  const long long W = amax + 1;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < words;
+       i += (long long)gridDim.x * blockDim.x) {
+    const int lane = (int)(i & 127);
+    long long t = i >> 7;
+    const int jq = (int)(t % Q4);
+    t /= Q4;
+    const int v = (int)(t % g.V);
+    t /= g.V;
+    const int m2f = (int)(t % N);
+    t /= N;
+    const int p = (int)(t % ML), k1f = (int)(t / ML);
+    const int k2f = lane / g.CL, c = lane - k2f * g.CL, l3f = v * g.CL + c;
+    float w[4] = {0.f, 0.f, 0.f, 0.f};
+    if (k2f < N && l3f < N && p < c32_nlist(N, k1f)) {
+      const int plo = k1f / 2;
+      const int l1f = p <= plo ? p : k1f + 1 + (p - plo - 1);
+      const int m1f = (k1f - l1f + N) % N, l2f = (k2f - m2f + N) % N;
+      // centred indices (FFTW index f -> (f + n) mod N) and modes (index - n)
+      const int l1 = (l1f + n) % N, l2 = (l2f + n) % N, l3 = (l3f + n) % N;
+      const int m1 = (m1f + n) % N, m2 = (m2f + n) % N;
+      const double sigmal = filter ? sigma[l1] * sigma[l2] * sigma[l3] : 1.0;
+      const double Bl = Bmm[((long long)l1 * N + l2) * N + l3];
+      for (int e = 0; e < 4; ++e) {
+        const int j = 4 * jq + e;
+        if (j >= N) continue;
+        const int m3 = ((j - v * g.CL + N) % N + n) % N;
+        const int x1 = l1 - n + m1 - n, x2 = l2 - n + m2 - n, x3 = l3 - n + m3 - n;
+        const int e1 = l1 - m1, e2 = l2 - m2, e3 = l3 - m3;
+        const int a = x1 * x1 + x2 * x2 + x3 * x3, b = e1 * e1 + e2 * e2 + e3 * e3;
+        const double sigmam = filter ? sigma[m1] * sigma[m2] * sigma[m3] : 1.0;
+        const double tv = T[(long long)a * W + b];
+        double y = tv * sigmal * sigmam * rval - Bmm[((long long)m1 * N + m2) * N + m3];
+        if (l1 != m1) y += tv * sigmam * sigmal * rval - Bl;
+        w[e] = (float)y;
+      }
+    }
+    out[i] = make_float4(w[0], w[1], w[2], w[3]);
+  }
+}
+
 edb_status launch_genB(int N, double gamma, double L, int filter, int mode, const double *d_T,
                        int amax, const double *d_sigma, const double *d_Bmm, double *d_B64,
                        float *d_B32, cudaStream_t st) {
@@ -285,8 +339,17 @@ edb_status launch_genB(int N, double gamma, double L, int filter, int mode, cons
   const double lam = lambda_pi();
   const double rval = (4. * M_PI) * pow(2. * lam / M_PI * L / N, 3 + gamma);
   long long NQ = (long long)N * N * N;
+  const bool tc = d_B32 && tc_takes(N);
+  if (tc) {
+    const long long words = c32_table_floats(N) / 4;
+    const long long blocks = std::min<long long>((words + 255) / 256, 64LL * device_sm_count());
+    genB32_tc_kernel<<<(unsigned)blocks, 256, 0, st>>>(N, filter, rval, d_T, amax, d_sigma, d_Bmm,
+                                                       tc_geom(N), words, (float4 *)d_B32);
+    EDB_LAUNCHED();
+    if (!d_B64) return EDB_OK;
+  }
   genB_kernel<<<(unsigned)NQ, 256, 0, st>>>(N, filter, rval, d_T, amax, d_sigma, d_Bmm, d_B64,
-                                            d_B32);
+                                            tc ? nullptr : d_B32);
   EDB_LAUNCHED();
   return EDB_OK;
 }

@@ -159,7 +159,8 @@ edb_status edb_qcalc_calQ_batch_f32_device(edb_qcalc *q, int S, const float *d_f
  * the result of each solve does not depend on S or the variant.  Without
  * chunks, variants 0-4 on the tensor-copy path (N % 4 == 0) run as one
  * persistent grid of resident CTAs pulling the work items from a queue (a
- * stream-ordered counter, so the call may be recorded into a graph). */
+ * stream-ordered counter, so the call may be recorded into a graph).  For
+ * N % 4 != 0 from 13 to 31 every variant is one and the same tensor-core launch. */
 edb_status edb_qcalc_calQ_batch_f32_ex(edb_qcalc *q, int S, int variant, int chunks,
                                        void *d_partial, const float *d_fin, float *d_Qout,
                                        void *stream);
