@@ -20,6 +20,17 @@
 // small fraction of its FP32 rate, and the FP64 passes of the batch's step
 // were bound by it (2.7 ms per pass at 4096 x N = 24).  Double-float keeps
 // about 2^-47 relative per operation.
+//
+// What little FP64 is left bounds a pass, so it is done once: the twiddles come
+// with the launch from the host (every block used to evaluate N sines and
+// cosines), and a dfc transform splits its input in the first pass, keeps
+// (hi, lo) pairs between the passes (the same 16 bytes) and joins them in the
+// last.  Transforms, us, before -> now (with N = 16, 24, 32 compiled in): 256 x
+// N = 16 185 -> 55 (dfc), 191 -> 115 (FP64), 92 -> 31 (FP32); 2048 x N = 24 3397 ->
+// 1280 (dfc).  A dfc pass that splits or joins still runs the FP64 pipe 75% busy.
+#include <math.h>
+
+#include <mutex>
 #include <type_traits>
 
 #include "edb_df.cuh"
@@ -154,6 +165,10 @@ __device__ __forceinline__ G from_work(R2 x, R scale) {
   return x;
 }
 template <>
+__device__ __forceinline__ dfc from_work<dfc, double, dfc>(dfc x, double) {
+  return x;  // between passes: no scale
+}
+template <>
 __device__ __forceinline__ double2 from_work<dfc, double, double2>(dfc x, double scale) {
   if (scale != 1.0) {
     const float2 sc = dsplit(scale);
@@ -162,15 +177,37 @@ __device__ __forceinline__ double2 from_work<dfc, double, double2>(dfc x, double
   return make_double2((double)x.rh + (double)x.rl, (double)x.ih + (double)x.il);
 }
 template <typename R2>
-__device__ __forceinline__ R2 make_tw(double c, double s) {
+R2 make_tw(double c, double s) {
   R2 w;
   w.x = (decltype(w.x))c;
   w.y = (decltype(w.y))s;
   return w;
 }
 template <>
-__device__ __forceinline__ dfc make_tw<dfc>(double c, double s) {
-  return mk_dfc(dsplit(c), dsplit(s));
+dfc make_tw<dfc>(double c, double s) {
+  const float ch = (float)c, sh = (float)s;
+  return dfc{ch, (float)(c - (double)ch), sh, (float)(s - (double)sh)};
+}
+// exp(sign 2 pi i r / N), r = 0 .. N - 1, passed to the kernel by value (so a
+// launch recorded into a graph carries it).
+constexpr int FFT_MAXN = 64;
+template <typename R2>
+struct FftTw {
+  R2 w[FFT_MAXN];
+};
+template <typename R2>
+const FftTw<R2> &fft_tw(int N, int sign) {
+  static std::once_flag once[FFT_MAXN + 1][2];
+  static FftTw<R2> tab[FFT_MAXN + 1][2];
+  const int s = sign > 0;
+  FftTw<R2> &t = tab[N][s];
+  std::call_once(once[N][s], [&] {
+    for (int r = 0; r < FFT_MAXN; ++r) {
+      const double ang = 8.0 * atan(1.0) * (r % N) / N;
+      t.w[r] = make_tw<R2>(cos(ang), sign * sin(ang));
+    }
+  });
+  return t;
 }
 
 // One Stockham stage of radix R (2, 3 or 4) on every line of the tile:
@@ -254,6 +291,20 @@ __device__ __forceinline__ void fft_stage_direct(int N, int LS, int Rd, int Ns, 
     dst[(size_t)line * LS + p] = o;
   }
 }
+// The stages of a size known at compile time, in fft_plan's order.
+template <int NC, int Ns, typename R2>
+__device__ __forceinline__ void fft_stages(int sign, R2 *&src, R2 *&dst, const R2 *tw) {
+  if constexpr (Ns < NC) {
+    constexpr int rem = NC / Ns, Rd = rem % 4 == 0 ? 4 : rem % 2 == 0 ? 2 : 3;
+    static_assert(rem % Rd == 0, "sizes of factors 2 and 3");
+    fft_stage_pow2<Rd>(NC, NC + 1, Ns, sign, src, dst, tw);
+    __syncthreads();
+    R2 *x = src;
+    src = dst;
+    dst = x;
+    fft_stages<NC, Ns * Rd>(sign, src, dst, tw);
+  }
+}
 }  // namespace
 
 // One pass: the tile's N lines along `axis` of cube blockIdx.y.
@@ -262,12 +313,15 @@ __device__ __forceinline__ void fft_stage_direct(int N, int LS, int Rd, int Ns, 
 //   axis 0: tile = rows i of fixed j (t); lines are columns (fixed k), along i.
 // Shared memory holds the tile twice (line stride N + 1, so that loading
 // columns does not hit one bank) and the twiddle table.  in may alias out
-// (passes 2 and 3 run in place): every global read happens before the first
-// barrier and every write after the last.
-template <typename R2, typename R, typename G>
-__global__ void fft_pass_kernel(int N, int axis, int sign, R scale, FftPlan plan, const G *in,
-                                G *out) {
+// (passes 2 and 3 run in place, element sizes equal): every global read happens
+// before the first barrier and every write after the last.
+// NC > 0: N known at compile time (the workloads' sizes): the stage loops'
+// divisions and remainders by N, N / R and Ns fold away.
+template <int NC, typename R2, typename R, typename GI, typename GO>
+__global__ void fft_pass_kernel(int n_, int axis, int sign, R scale, FftPlan plan,
+                                const __grid_constant__ FftTw<R2> twt, const GI *in, GO *out) {
   extern __shared__ unsigned char smem_raw[];
+  const int N = NC > 0 ? NC : n_;
   const int LS = N + 1;
   R2 *buf0 = reinterpret_cast<R2 *>(smem_raw);  // [N][LS]
   R2 *buf1 = buf0 + (size_t)N * LS;              // [N][LS]
@@ -287,20 +341,18 @@ __global__ void fft_pass_kernel(int N, int axis, int sign, R scale, FftPlan plan
   // tile element (u, v): u = row, v = column (contiguous in memory)
   for (int e = threadIdx.x; e < N * N; e += blockDim.x) {
     const int u = e / N, v = e - u * N;
-    const R2 x = to_work<R2, G>(in[base + (long long)u * row_stride + v]);
+    const R2 x = to_work<R2, GI>(in[base + (long long)u * row_stride + v]);
     if (axis == 2)
       buf0[(size_t)u * LS + v] = x;
     else
       buf0[(size_t)v * LS + u] = x;
   }
-  for (int r = threadIdx.x; r < N; r += blockDim.x) {
-    const double ang = 8.0 * atan(1.0) * r / N;
-    tw[r] = make_tw<R2>(cos(ang), sign * sin(ang));
-  }
+  for (int r = threadIdx.x; r < N; r += blockDim.x) tw[r] = twt.w[r];
   __syncthreads();
   R2 *src = buf0, *dst = buf1;
+  if constexpr (NC > 0) fft_stages<NC, 1>(sign, src, dst, tw);
   int Ns = 1;
-  for (int s = 0; s < plan.nst; ++s) {
+  for (int s = 0; NC == 0 && s < plan.nst; ++s) {
     const int Rd = plan.radix[s];
     if (Rd == 4)
       fft_stage_pow2<4>(N, LS, Ns, sign, src, dst, tw);
@@ -319,31 +371,50 @@ __global__ void fft_pass_kernel(int N, int axis, int sign, R scale, FftPlan plan
   for (int e = threadIdx.x; e < N * N; e += blockDim.x) {
     const int u = e / N, v = e - u * N;
     const R2 x = (axis == 2) ? src[(size_t)u * LS + v] : src[(size_t)v * LS + u];
-    out[base + (long long)u * row_stride + v] = from_work<R2, R, G>(x, scale);
+    out[base + (long long)u * row_stride + v] = from_work<R2, R, GO>(x, scale);
   }
 }
 
-template <typename R2, typename R, typename G>
-static edb_status dft3d_t(int N, int batch, const G *in, G *out, int inverse, cudaStream_t st) {
-  if (N < 1 || N > 64) return fail(EDB_EINVAL, "dft3d: N out of range [1,64]");
-  const int sign = inverse ? +1 : -1;
+template <int NC, typename R2, typename R, typename GI, typename GO>
+static edb_status fft_pass_n(int N, int batch, int axis, int sign, R scale, const FftPlan &plan,
+                           const GI *in, GO *out, cudaStream_t st) {
+  static_assert(sizeof(GI) == sizeof(GO), "passes run in place");
+  auto kern = fft_pass_kernel<NC, R2, R, GI, GO>;
+  // once per instantiation, thread-safe (N = 64 in FP64 needs 131 KB)
+  static const cudaError_t configured =
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+  if (configured != cudaSuccess) return cuda_fail(configured, "cudaFuncSetAttribute(fft_pass)");
   const int threads = N * N < FFT_THREADS ? ((N * N + 31) / 32) * 32 : FFT_THREADS;
   const size_t smem = sizeof(R2) * (2 * (size_t)N * (N + 1) + N);
-  // once per instantiation, thread-safe (N = 64 in FP64 needs 131 KB)
-  static const cudaError_t configured = cudaFuncSetAttribute(
-      fft_pass_kernel<R2, R, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-  if (configured != cudaSuccess) return cuda_fail(configured, "cudaFuncSetAttribute(fft_pass)");
-  const FftPlan plan = fft_plan(N);
-  dim3 grid((unsigned)N, (unsigned)batch);
-  const R one = (R)1;
-  const R scale = inverse ? (R)(1. / ((double)N * N * N)) : one;
-  fft_pass_kernel<R2, R, G><<<grid, threads, smem, st>>>(N, 2, sign, one, plan, in, out);
-  EDB_LAUNCHED();
-  fft_pass_kernel<R2, R, G><<<grid, threads, smem, st>>>(N, 1, sign, one, plan, out, out);
-  EDB_LAUNCHED();
-  fft_pass_kernel<R2, R, G><<<grid, threads, smem, st>>>(N, 0, sign, scale, plan, out, out);
+  kern<<<dim3((unsigned)N, (unsigned)batch), threads, smem, st>>>(N, axis, sign, scale, plan,
+                                                                  fft_tw<R2>(N, sign), in, out);
   EDB_LAUNCHED();
   return EDB_OK;
+}
+
+template <typename R2, typename R, typename GI, typename GO>
+static edb_status fft_pass(int N, int batch, int axis, int sign, R scale, const FftPlan &plan,
+                           const GI *in, GO *out, cudaStream_t st) {
+  switch (N) {
+    case 16: return fft_pass_n<16, R2, R, GI, GO>(N, batch, axis, sign, scale, plan, in, out, st);
+    case 24: return fft_pass_n<24, R2, R, GI, GO>(N, batch, axis, sign, scale, plan, in, out, st);
+    case 32: return fft_pass_n<32, R2, R, GI, GO>(N, batch, axis, sign, scale, plan, in, out, st);
+    default: return fft_pass_n<0, R2, R, GI, GO>(N, batch, axis, sign, scale, plan, in, out, st);
+  }
+}
+
+// R2: working type, also the memory type between the passes.
+template <typename R2, typename R, typename G>
+static edb_status dft3d_t(int N, int batch, const G *in, G *out, int inverse, cudaStream_t st) {
+  if (N < 1 || N > FFT_MAXN) return fail(EDB_EINVAL, "dft3d: N out of range [1,64]");
+  const int sign = inverse ? +1 : -1;
+  const FftPlan plan = fft_plan(N);
+  const R one = (R)1;
+  const R scale = inverse ? (R)(1. / ((double)N * N * N)) : one;
+  R2 *mid = reinterpret_cast<R2 *>(out);
+  EDB_TRY((fft_pass<R2, R, G, R2>(N, batch, 2, sign, one, plan, in, mid, st)));
+  EDB_TRY((fft_pass<R2, R, R2, R2>(N, batch, 1, sign, one, plan, mid, mid, st)));
+  return fft_pass<R2, R, R2, G>(N, batch, 0, sign, scale, plan, mid, out, st);
 }
 
 edb_status launch_dft3d(int N, int batch, const void *d_in, void *d_out, void *d_tmp, int inverse,
