@@ -293,38 +293,69 @@ edb_status launch_efix_fixsol(int Nf, double *d_f, EfixState *d_state, double ep
 //   STAGE_SSP3_3  y = x/3. + 2.*z/3. + c1*q0         SSP3 :423-424
 //   STAGE_RK4     y = x + c1*(q0 + 2.*q1 + 2.*q2 + q3)   RK4 :493-494
 //   STAGE_DUFORT  y = c0*(z + c1*q0 + c2*(z - w))    DUFORT :597-598
-// Q-hat inputs are double2 (FP64 path) or float2 (batched FP32 path, widened
-// exactly).  y32, when given, receives the result rounded to float.
-template <typename TQ>
-__device__ __forceinline__ double2 ld(const TQ *p, long long i) {
-  return make_double2((double)p[i].x, (double)p[i].y);
+// y32, when given, receives the result rounded to float.
+
+// The batch's updates (FP32 Q-hat) with fused multiply-adds, each with fewer
+// roundings than the reference's expression; its FP64 arithmetic, not its bytes,
+// bounds this kernel.  x / 3 is x times 1/3 as an unevaluated sum of two doubles.
+// 256 solves of N = 16, expression by expression as below -> here: AXPY 19.6 ->
+// 16.1 us, SSP3 31.6 -> 24.2 and 90 -> 28.0.
+__device__ __forceinline__ double third(double x) {
+  const double hi = 1. / 3., lo = 0x1.5555555555555p-56;  // hi + lo = 1/3 to 2^-108
+  return __fma_rn(x, hi, x * lo);
+}
+__device__ __forceinline__ double stage_f32(int op, double c1, double a, double b, double q0,
+                                            double q1, double q2, double q3) {
+  if (op == STAGE_AXPY) return __fma_rn(c1, q0, a);
+  if (op == STAGE_SSP3_2) return __fma_rn(c1, q0, __fma_rn(0.25, b, 0.75 * a));
+  if (op == STAGE_SSP3_3) return __fma_rn(c1, q0, third(__fma_rn(2., b, a)));
+  return __fma_rn(c1, __fma_rn(2., q2, __fma_rn(2., q1, q0)) + q3, a);  // STAGE_RK4
+}
+__global__ void stage_f32q_kernel(long long n, int op, double c1, double2 *y, const double2 *x,
+                                  const double2 *z, const float2 *q0, const float2 *q1,
+                                  const float2 *q2, const float2 *q3, float2 *y32) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const bool two = op == STAGE_SSP3_2 || op == STAGE_SSP3_3;
+  const double2 a = x[i], b = two ? z[i] : make_double2(0., 0.);
+  const float2 p0 = q0[i];
+  float2 p1 = p0, p2 = p0, p3 = p0;
+  if (op == STAGE_RK4) {
+    p1 = q1[i];
+    p2 = q2[i];
+    p3 = q3[i];
+  }
+  const double rx = stage_f32(op, c1, a.x, b.x, p0.x, p1.x, p2.x, p3.x);
+  const double ry = stage_f32(op, c1, a.y, b.y, p0.y, p1.y, p2.y, p3.y);
+  if (y) y[i] = make_double2(rx, ry);
+  if (y32) y32[i] = make_float2((float)rx, (float)ry);
 }
 
-template <typename TQ>
 __global__ void stage_kernel(long long n, int op, double c0, double c1, double c2, double2 *y,
-                             const double2 *x, const double2 *z, const double2 *w, const TQ *q0,
-                             const TQ *q1, const TQ *q2, const TQ *q3, float2 *y32) {
+                             const double2 *x, const double2 *z, const double2 *w,
+                             const double2 *q0, const double2 *q1, const double2 *q2,
+                             const double2 *q3, float2 *y32) {
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   double rx, ry;
   if (op == STAGE_AXPY) {
-    double2 a = x[i], q = ld(q0, i);
+    double2 a = x[i], q = q0[i];
     rx = a.x + c1 * q.x;
     ry = a.y + c1 * q.y;
   } else if (op == STAGE_SSP3_2) {
-    double2 a = x[i], b = z[i], q = ld(q0, i);
+    double2 a = x[i], b = z[i], q = q0[i];
     rx = 0.75 * a.x + 0.25 * b.x + c1 * q.x;
     ry = 0.75 * a.y + 0.25 * b.y + c1 * q.y;
   } else if (op == STAGE_SSP3_3) {
-    double2 a = x[i], b = z[i], q = ld(q0, i);
+    double2 a = x[i], b = z[i], q = q0[i];
     rx = a.x / 3. + 2. * b.x / 3. + c1 * q.x;
     ry = a.y / 3. + 2. * b.y / 3. + c1 * q.y;
   } else if (op == STAGE_RK4) {
-    double2 a = x[i], p0 = ld(q0, i), p1 = ld(q1, i), p2 = ld(q2, i), p3 = ld(q3, i);
+    double2 a = x[i], p0 = q0[i], p1 = q1[i], p2 = q2[i], p3 = q3[i];
     rx = a.x + c1 * (p0.x + 2. * p1.x + 2. * p2.x + p3.x);
     ry = a.y + c1 * (p0.y + 2. * p1.y + 2. * p2.y + p3.y);
   } else {  // STAGE_DUFORT
-    double2 b = z[i], o = w[i], q = ld(q0, i);
+    double2 b = z[i], o = w[i], q = q0[i];
     rx = c0 * (b.x + c1 * q.x + c2 * (b.x - o.x));
     ry = c0 * (b.y + c1 * q.y + c2 * (b.y - o.y));
   }
@@ -332,29 +363,28 @@ __global__ void stage_kernel(long long n, int op, double c0, double c1, double c
   if (y32) y32[i] = make_float2((float)rx, (float)ry);
 }
 
-template <typename TQ>
-static edb_status stage_t(long long n, int op, double c0, double c1, double c2, double2 *y,
-                          const double2 *x, const double2 *z, const double2 *w, const TQ *q0,
-                          const TQ *q1, const TQ *q2, const TQ *q3, float2 *y32,
-                          cudaStream_t st) {
-  stage_kernel<TQ><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(n, op, c0, c1, c2, y, x, z, w,
-                                                                 q0, q1, q2, q3, y32);
-  EDB_LAUNCHED();
-  return EDB_OK;
-}
-
 edb_status launch_stage(long long n, int op, double c0, double c1, double c2, double2 *y,
                         const double2 *x, const double2 *z, const double2 *w, const double2 *q0,
                         const double2 *q1, const double2 *q2, const double2 *q3, float2 *y32,
                         cudaStream_t st) {
-  return stage_t<double2>(n, op, c0, c1, c2, y, x, z, w, q0, q1, q2, q3, y32, st);
+  stage_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(n, op, c0, c1, c2, y, x, z, w, q0, q1,
+                                                            q2, q3, y32);
+  EDB_LAUNCHED();
+  return EDB_OK;
 }
 
 edb_status launch_stage_f32q(long long n, int op, double c0, double c1, double c2, double2 *y,
                              const double2 *x, const double2 *z, const double2 *w,
                              const float2 *q0, const float2 *q1, const float2 *q2,
                              const float2 *q3, float2 *y32, cudaStream_t st) {
-  return stage_t<float2>(n, op, c0, c1, c2, y, x, z, w, q0, q1, q2, q3, y32, st);
+  (void)c0;
+  (void)c2;
+  (void)w;
+  if (op == STAGE_DUFORT) return fail(EDB_EINVAL, "stage: no FP32 form of DUFORT");
+  stage_f32q_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(n, op, c1, y, x, z, q0, q1, q2,
+                                                                 q3, y32);
+  EDB_LAUNCHED();
+  return EDB_OK;
 }
 
 __global__ void d2f_kernel(long long n, const double2 *x, float2 *y) {
