@@ -656,7 +656,7 @@ static edb_status multi_inputs(int ntab, edb_qcalc *const *qs, const int *S,
       heaviest = work;
       bool tuned = false;
       const int v = qcalc_c32_variant(qs[i], S[i], &tuned, false);
-      *auto_variant = !tuned ? 4 : (calq32_pair(v) ? v - 5 : v);
+      *auto_variant = !tuned || v > 9 ? 4 : (calq32_pair(v) ? v - 5 : v);
     }
   }
   return EDB_OK;
@@ -670,6 +670,7 @@ extern "C" edb_status edb_qcalc_calQ_batch_multi(int ntab, edb_qcalc *const *qs,
   int v = 4;
   EDB_TRY(multi_inputs(ntab, qs, S, d_fin, d_Qout, in, &v));
   if (variant >= 0) v = variant;
+  if (v > 4) return fail(EDB_EINVAL, "calq32 multi: a plain-layout variant (0-4)");
   return launch_calq32_multi(ntab, in, v, (cudaStream_t)stream);
 }
 
@@ -689,7 +690,7 @@ extern "C" edb_status edb_qcalc_autotune_batch_multi(int ntab, edb_qcalc *const 
   float best_ms = 1e30f;
   edb_status rc = EDB_OK;
   for (int v = 0; v < calq32_variants() && rc == EDB_OK; ++v) {
-    if (calq32_pair(v)) continue;
+    if (v > 4) break;  // the plain-layout variants of 16- and 4-solve groups
     rc = launch_calq32_multi(ntab, in, v, st);  // warm-up; EINVAL: does not fit
     if (rc == EDB_EINVAL) {
       rc = EDB_OK;

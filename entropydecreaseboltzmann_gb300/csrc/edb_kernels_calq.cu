@@ -238,7 +238,7 @@ edb_status launch_calq64_reduce(const QParams &p, int nchunk, const double2 *d_p
 // is in the batch.
 // ---------------------------------------------------------------------------
 namespace {
-constexpr int SC = 2;                     // solves per thread: w and w + WS
+constexpr int SC = 2;                     // solves per thread: w and w + WS (variants 10, 11: 1)
 constexpr int ROWPAD = 8;                 // floats after each B-tile row
 constexpr int FLPAD = 2;                  // complex after each f_l line
 constexpr int PLPAD = 2;                  // complex after each solve's plane
@@ -711,14 +711,19 @@ __device__ __forceinline__ void compute_line_pair(const C32Geom &g, const float 
 // compute_line_al_n); the line's RC groups are then unrolled, so loads of one
 // group are scheduled under the arithmetic of the one before (4096 x N = 24:
 // 104 -> 99 ms).
-template <int A, int RC = 0>
+template <int A, int RC, int SN>
 __device__ __forceinline__ void compute_line_al(const C32Geom &g, const float *Bt,
                                                 const float2 *fl0, const float2 *fl1,
                                                 const float2 *p0, const float2 *p1, int k3_0,
-                                                u64 (&accA)[A][SC], u64 (&accB)[A][SC]) {
+                                                u64 (&accA)[A][SN], u64 (&accB)[A][SN]) {
   const int N = RC > 0 ? RC * A : g.N;
-  const uint32_t sp0 = s_addr(p0), sp1 = s_addr(p1);
-  uint32_t sf0 = s_addr(fl0), sf1 = s_addr(fl1), bB = s_addr(Bt);
+  uint32_t sp[SN], sf[SN], bB = s_addr(Bt);
+  sp[0] = s_addr(p0);
+  sf[0] = s_addr(fl0);
+  if constexpr (SN == 2) {
+    sp[1] = s_addr(p1);
+    sf[1] = s_addr(fl1);
+  }
   const uint32_t brow = 4u * g.BROW;
   // f-hat values move in 16-byte pairs: every plane row, line and stage
   // offset is an even number of complex values here (N % 4 == 0, even
@@ -726,42 +731,40 @@ __device__ __forceinline__ void compute_line_al(const C32Geom &g, const float *B
   // hit 8 distinct 16-byte bank groups (plane pitch N^2 + 2 complex = an odd
   // number of pairs), where single-value loads of two windows 4 apart met
   // pairwise in the same banks.
-  u64 ring[A][SC];
-  {
-    const uint32_t a0 = sp0 + 8u * k3_0, a1 = sp1 + 8u * k3_0;
+  u64 ring[A][SN];
 #pragma unroll
-    for (int a = 0; a < A; a += 2) {
-      const ulonglong2 v0 = lds_u64x2(a0 + 8u * a), v1 = lds_u64x2(a1 + 8u * a);
-      ring[a][0] = v0.x;
-      ring[a + 1][0] = v0.y;
-      ring[a][1] = v1.x;
-      ring[a + 1][1] = v1.y;
+  for (int a = 0; a < A; a += 2)
+#pragma unroll
+    for (int c = 0; c < SN; ++c) {
+      const ulonglong2 v = lds_u64x2(sp[c] + 8u * (k3_0 + a));
+      ring[a][c] = v.x;
+      ring[a + 1][c] = v.y;
     }
-  }
-  u64 held[SC] = {0ull, 0ull};  // f_m at qq - t for the next even step (or next group's t = 0)
+  u64 held[SN];  // f_m at qq - t for the next even step (or next group's t = 0)
+#pragma unroll
+  for (int c = 0; c < SN; ++c) held[c] = 0ull;
   int base = k3_0;
 #pragma unroll(RC > 0 ? RC : 1)
   for (int gg = 0; gg < (RC > 0 ? RC : g.R); ++gg) {
     const int qq = base == 0 ? N : base;
-    const uint32_t qa = sp0 + 8u * qq, qb = sp1 + 8u * qq;
-    ulonglong2 fp0 = make_ulonglong2(0ull, 0ull), fp1 = fp0;  // f_l of steps (t, t + 1)
+    ulonglong2 fp[SN];  // f_l of steps (t, t + 1)
 #pragma unroll
     for (int t = 0; t < A; ++t) {
       // the ring entry of step t: f_m at qq - t (t = 0: base, held over)
       if (t == 0) {
-        if (gg > 0) {
-          ring[0][0] = held[0];
-          ring[0][1] = held[1];
-        }
+        if (gg > 0)
+#pragma unroll
+          for (int c = 0; c < SN; ++c) ring[0][c] = held[c];
       } else if (t & 1) {  // pair (qq - t - 1, qq - t)
-        const ulonglong2 v0 = lds_u64x2(qa - 8u * (t + 1)), v1 = lds_u64x2(qb - 8u * (t + 1));
-        ring[(A - t) % A][0] = v0.y;
-        ring[(A - t) % A][1] = v1.y;
-        held[0] = v0.x;
-        held[1] = v1.x;
+#pragma unroll
+        for (int c = 0; c < SN; ++c) {
+          const ulonglong2 v = lds_u64x2(sp[c] + 8u * qq - 8u * (t + 1));
+          ring[(A - t) % A][c] = v.y;
+          held[c] = v.x;
+        }
       } else {
-        ring[(A - t) % A][0] = held[0];
-        ring[(A - t) % A][1] = held[1];
+#pragma unroll
+        for (int c = 0; c < SN; ++c) ring[(A - t) % A][c] = held[c];
       }
       float bv[A];
 #pragma unroll
@@ -773,27 +776,28 @@ __device__ __forceinline__ void compute_line_al(const C32Geom &g, const float *B
         bv[4 * q4 + 3] = b.w;
       }
       bB += brow;
-      if ((t & 1) == 0) {
-        fp0 = lds_u64x2(sf0 + 8u * t);
-        fp1 = lds_u64x2(sf1 + 8u * t);
+      u64 flx[SN], fly[SN];
+#pragma unroll
+      for (int c = 0; c < SN; ++c) {
+        if ((t & 1) == 0) fp[c] = lds_u64x2(sf[c] + 8u * t);
+        const float2 f = upk((t & 1) ? fp[c].y : fp[c].x);
+        flx[c] = pk(f.x, f.x);
+        fly[c] = pk(f.y, f.y);
       }
-      const float2 f0 = upk((t & 1) ? fp0.y : fp0.x), f1 = upk((t & 1) ? fp1.y : fp1.x);
-      const u64 flx[SC] = {pk(f0.x, f0.x), pk(f1.x, f1.x)};
-      const u64 fly[SC] = {pk(f0.y, f0.y), pk(f1.y, f1.y)};
 #pragma unroll
       for (int a = 0; a < A; ++a) {
         const int slot = (a - t + A) % A;
         const u64 bb = pk(bv[a], bv[a]);
 #pragma unroll
-        for (int c = 0; c < SC; ++c) {
+        for (int c = 0; c < SN; ++c) {
           const u64 q = mul2(bb, ring[slot][c]);
           fma2(accA[a][c], flx[c], q);
           fma2(accB[a][c], fly[c], q);
         }
       }
     }
-    sf0 += 8u * A;
-    sf1 += 8u * A;
+#pragma unroll
+    for (int c = 0; c < SN; ++c) sf[c] += 8u * A;
     base -= A;
     if (base < 0) base += N;
   }
@@ -855,19 +859,19 @@ __device__ __forceinline__ void compute_line_pair_al(const C32Geom &g, const flo
 // The aligned lines with N fixed at compile time for the workload sizes
 // N = 16, 24, 32 (the serving mix and the uniform batch), generic otherwise.
 // The branch is uniform over the CTA.
-template <int A>
+template <int A, int SN>
 __device__ __forceinline__ void compute_line_al_n(const C32Geom &g, const float *Bt,
                                                   const float2 *fl0, const float2 *fl1,
                                                   const float2 *p0, const float2 *p1, int k3_0,
-                                                  u64 (&accA)[A][SC], u64 (&accB)[A][SC]) {
+                                                  u64 (&accA)[A][SN], u64 (&accB)[A][SN]) {
   if (g.N == 24)
-    compute_line_al<A, 24 / A>(g, Bt, fl0, fl1, p0, p1, k3_0, accA, accB);
+    compute_line_al<A, 24 / A, SN>(g, Bt, fl0, fl1, p0, p1, k3_0, accA, accB);
   else if (g.N == 32)
-    compute_line_al<A, 32 / A>(g, Bt, fl0, fl1, p0, p1, k3_0, accA, accB);
+    compute_line_al<A, 32 / A, SN>(g, Bt, fl0, fl1, p0, p1, k3_0, accA, accB);
   else if (g.N == 16)
-    compute_line_al<A, 16 / A>(g, Bt, fl0, fl1, p0, p1, k3_0, accA, accB);
+    compute_line_al<A, 16 / A, SN>(g, Bt, fl0, fl1, p0, p1, k3_0, accA, accB);
   else
-    compute_line_al<A>(g, Bt, fl0, fl1, p0, p1, k3_0, accA, accB);
+    compute_line_al<A, 0, SN>(g, Bt, fl0, fl1, p0, p1, k3_0, accA, accB);
 }
 template <int A>
 __device__ __forceinline__ void compute_line_pair_al_n(const C32Geom &g, const float *Bt,
@@ -911,7 +915,7 @@ __global__ void c32_pairs_kernel(int S, long long NQ, const float2 *__restrict__
 // groups x chunks, N, k2 tiles) CTAs over one table (see calq32_kernel).
 // Returns false when a bounded wait ran out (the CTA drained its copies and
 // set the status word); every thread returns at the same point.
-template <bool TMA, int MAXT, bool HLS, int WS, int A, int MINB, bool PAIR>
+template <bool TMA, int MAXT, bool HLS, int WS, int A, int MINB, bool PAIR, int SN>
 __device__ __forceinline__ bool calq32_cta(int N, int S, int K2T, int NST, int NPL, int C, int GB,
                                            const float *__restrict__ B32,
                                            const float2 *__restrict__ fin,
@@ -919,6 +923,7 @@ __device__ __forceinline__ bool calq32_cta(int N, int S, int K2T, int NST, int N
                                            int tmap, unsigned long long wait_ns,
                                            const CUtensorMap *tmB, const CUtensorMap *tmF, int U,
                                            int GY, int GZ, long long lin, int nthr) {
+  constexpr int SC = SN;       // solves per thread: w and, with two, w + WS
   constexpr int SG = SC * WS;  // solves per group
   extern __shared__ __align__(128) unsigned char smem[];
   const C32Geom g =
@@ -1106,7 +1111,11 @@ __device__ __forceinline__ bool calq32_cta(int N, int S, int K2T, int NST, int N
     const float *Bt = Bs + (size_t)st * g.BSTG + k2l * N + k3_0;
     const float2 *fl0 = fls + (size_t)st * g.FSTG + (size_t)w * g.FLS;
     const float2 *p0 = plb + (size_t)pb * plane_sz + (size_t)w * g.PSTR + m2 * N * g.EL;
-    if (PAIR) {
+    const float2 *fl1 = fl0 + (size_t)WS * g.FLS;
+    const float2 *p1 = p0 + (size_t)WS * g.PSTR;
+    if constexpr (SC == 1) {  // tensor-copy path with N % A == 0 only (see the launcher)
+      compute_line_al_n<A, 1>(g, Bt, fl0, fl1, p0, p1, k3_0, accA, accB);
+    } else if constexpr (PAIR) {
       if (TMA && ring_al && FIXN)
         compute_line_pair_al_n<A>(g, Bt, fl0, p0, k3_0, accA, accB);
       else if (TMA && ring_al)
@@ -1116,12 +1125,10 @@ __device__ __forceinline__ bool calq32_cta(int N, int S, int K2T, int NST, int N
       else
         compute_line_pair<false, false, A>(g, Bt, fl0, p0, k3_0, accA, accB);
     } else {
-      const float2 *fl1 = fl0 + (size_t)WS * g.FLS;
-      const float2 *p1 = p0 + (size_t)WS * g.PSTR;
       if (TMA && ring_al && FIXN)
-        compute_line_al_n<A>(g, Bt, fl0, fl1, p0, p1, k3_0, accA, accB);
+        compute_line_al_n<A, 2>(g, Bt, fl0, fl1, p0, p1, k3_0, accA, accB);
       else if (TMA && ring_al)
-        compute_line_al<A>(g, Bt, fl0, fl1, p0, p1, k3_0, accA, accB);
+        compute_line_al<A, 0, 2>(g, Bt, fl0, fl1, p0, p1, k3_0, accA, accB);
       else if (TMA)
         compute_line<true, true, A>(g, Bt, fl0, fl1, p0, p1, k3_0, accA, accB);
       else
@@ -1143,8 +1150,10 @@ __device__ __forceinline__ bool calq32_cta(int N, int S, int K2T, int NST, int N
         u64 xs[SC];
 #pragma unroll
         for (int c = 0; c < SC; ++c)
-          xs[c] = !PAIR ? fma2r(neg_re, swp(accB[a][c]), accA[a][c])
-                  : c == 0 ? fma2r(neg_one, accB[a][1], accA[a][0])
+          if constexpr (!PAIR)
+            xs[c] = fma2r(neg_re, swp(accB[a][c]), accA[a][c]);
+          else
+            xs[c] = c == 0 ? fma2r(neg_one, accB[a][1], accA[a][0])
                            : add2(accA[a][1], accB[a][0]);
 #pragma unroll
         for (int c = 0; c < SC; ++c) {
@@ -1231,7 +1240,7 @@ __device__ __forceinline__ bool calq32_cta(int N, int S, int K2T, int NST, int N
           }
         }
         float2 h, l;
-        if (PAIR) {
+        if constexpr (PAIR) {
           const float2 hr = upk(hv[0]), hm = upk(hv[1]), lr = upk(lv[0]), lm = upk(lv[1]);
           h = c == 0 ? make_float2(hr.x, hm.x) : make_float2(hr.y, hm.y);
           l = c == 0 ? make_float2(lr.x, lm.x) : make_float2(lr.y, lm.y);
@@ -1259,7 +1268,7 @@ __global__ void __launch_bounds__(MAXT, MINB)
                   const __grid_constant__ CUtensorMap tmF) {
   const long long lin =
       blockIdx.x + (long long)gridDim.x * (blockIdx.y + (long long)gridDim.y * blockIdx.z);
-  calq32_cta<TMA, MAXT, HLS, WS, A, MINB, PAIR>(N, S, K2T, NST, NPL, C, GB, B32, fin, Q, partial,
+  calq32_cta<TMA, MAXT, HLS, WS, A, MINB, PAIR, 2>(N, S, K2T, NST, NPL, C, GB, B32, fin, Q, partial,
                                                tmap, wait_ns, &tmB, &tmF, gridDim.x, gridDim.y,
                                                gridDim.z, lin, (int)blockDim.x);
 }
@@ -1288,7 +1297,7 @@ struct C32Multi {
   unsigned long long *queue;  // next item, zero at launch; null: item b + k gridDim.x
 };
 
-template <bool TMA, int MAXT, bool HLS, int WS, int A, int MINB, bool PAIR>
+template <bool TMA, int MAXT, bool HLS, int WS, int A, int MINB, bool PAIR, int SN>
 __global__ void __launch_bounds__(MAXT, MINB)
     calq32_multi_kernel(const __grid_constant__ C32Multi mt, unsigned long long wait_ns) {
   extern __shared__ __align__(128) unsigned char smem[];
@@ -1309,7 +1318,7 @@ __global__ void __launch_bounds__(MAXT, MINB)
     int t = 0;
     while (t + 1 < mt.ntab && item >= mt.t[t + 1].begin) ++t;
     const C32Table &d = mt.t[t];
-    const bool ok = calq32_cta<TMA, MAXT, HLS, WS, A, MINB, PAIR>(
+    const bool ok = calq32_cta<TMA, MAXT, HLS, WS, A, MINB, PAIR, SN>(
         d.N, d.S, d.K2T, d.NST, d.NPL, d.C, d.GB, d.B32, d.fin, d.Q, d.partial, d.tmap, wait_ns,
         &d.tmB, &d.tmF, d.U, d.GY, d.GZ, item - d.begin, d.threads);
     if (!ok) break;  // uniform: the CTA drained its copies and set the status word
@@ -1350,19 +1359,25 @@ __global__ void calq32_reduce_kernel(long long n, int C, const float4 *__restric
 //   4: WS 8, A 4, <= 384 threads, registers (<= 168 registers)
 //   5-9: 0-4 on the solve-pair layout (same bits, fewer operand moves and
 //        shared-memory loads; needs a pair-layout copy of the input)
+//   10: WS 4, A 4, one solve a thread (4-solve groups), <= 256 threads
+//   11: WS 2, the same (2-solve groups)
+// 10 and 11 are for the few solves that leave 16-solve lanes empty: TIMING_S
 struct C32Variant {
   int ws, a, maxt;
   bool hls;
   int minb;
   bool pair;
+  int sc;  // solves per thread
 };
 constexpr C32Variant kC32Variants[] = {
-    {8, 8, 256, false, 1, false}, {8, 8, 384, true, 1, false}, {2, 8, 256, false, 1, false},
-    {8, 4, 256, false, 2, false}, {8, 4, 384, false, 1, false}, {8, 8, 256, false, 1, true},
-    {8, 8, 384, true, 1, true},   {2, 8, 256, false, 1, true},  {8, 4, 256, false, 2, true},
-    {8, 4, 384, false, 1, true}};
+    {8, 8, 256, false, 1, false, 2}, {8, 8, 384, true, 1, false, 2},
+    {2, 8, 256, false, 1, false, 2}, {8, 4, 256, false, 2, false, 2},
+    {8, 4, 384, false, 1, false, 2}, {8, 8, 256, false, 1, true, 2},
+    {8, 8, 384, true, 1, true, 2},   {2, 8, 256, false, 1, true, 2},
+    {8, 4, 256, false, 2, true, 2},  {8, 4, 384, false, 1, true, 2},
+    {4, 4, 256, false, 2, false, 1}, {2, 4, 256, false, 2, false, 1}};
 int calq32_variants() { return (int)(sizeof(kC32Variants) / sizeof(kC32Variants[0])); }
-int calq32_group(int variant) { return SC * kC32Variants[variant].ws; }
+int calq32_group(int variant) { return kC32Variants[variant].sc * kC32Variants[variant].ws; }
 bool calq32_pair(int variant) { return kC32Variants[variant].pair; }
 size_t calq32_pair_bytes(int N, int S) { return (size_t)((S + 1) / 2) * N * N * N * sizeof(float4); }
 
@@ -1455,11 +1470,17 @@ struct C32Setup {
 static edb_status c32_setup(int N, int S, const C32Variant &vr, int C, const float *d_B32,
                             const float2 *src, int block_threads, C32Setup *o) {
   const int maxt = vr.maxt, WS = vr.ws, A = vr.a;
-  const int SG = SC * WS;
+  const int SG = vr.sc * WS;
   const int R = (N + A - 1) / A;
   int K2T = maxt / (R * WS);
   if (K2T > N) K2T = N;
   if (K2T < 1) return fail(EDB_EINVAL, "calq32: N too large for the thread tile");
+  // few solves: smaller tiles (to one warp) until there are two CTAs an SM
+  if (vr.sc == 1)
+    while (K2T > 1 && (K2T / 2) * R * WS >= 32 &&
+           (long long)((S + SG - 1) / SG) * C * N * ((N + K2T - 1) / K2T) <
+               2LL * device_sm_count())
+      K2T /= 2;
   const int tiles = (N + K2T - 1) / K2T;
   K2T = (N + tiles - 1) / tiles;
   o->K2T = K2T;
@@ -1543,13 +1564,22 @@ edb_status launch_calq32_batch(int N, int S, const float *d_B32, const float2 *d
     EDB_TRY(launch_calqtc(N, S, d_B32, d_fin, d_Q, C, d_partial, st));
     return C == 1 ? EDB_OK : launch_c32_reduce(N, S, C, d_partial, d_Q, st);
   }
+  // the one-solve variants have no plain-load form: others give the same bits
+  if (kC32Variants[variant].sc == 1) {
+    C32Setup su;
+    if (N % kC32Variants[variant].a ||
+        c32_setup(N, S, kC32Variants[variant], C, d_B32, d_fin, 0, &su) != EDB_OK || !su.tma ||
+        !su.maps.tmap)
+      variant = 0;
+  }
   const C32Variant &vr = kC32Variants[variant];
   if (vr.pair && !d_pairs) return fail(EDB_EINVAL, "calq32: pair variants need a pair buffer");
-  const int SG = SC * vr.ws;
+  const int SG = vr.sc * vr.ws;
   const float2 *src = vr.pair ? reinterpret_cast<const float2 *>(d_pairs) : d_fin;
   C32Setup su;
   EDB_TRY(c32_setup(N, S, vr, C, d_B32, src, 0, &su));
-  if (!vr.pair && su.tma && su.maps.tmap && (persist > 0 || (persist < 0 && C == 1))) {
+  if (!vr.pair && su.tma && su.maps.tmap &&
+      (persist > 0 || (persist < 0 && C == 1) || vr.sc == 1)) {
     // one persistent grid of resident CTAs pulls the launch's CTA work items
     // from a queue, in the launch's order (same CTA work, so the same bits;
     // 4096 x N = 24: 84.9 -> 83.0 ms).  Taken round-robin instead, the items
@@ -1558,7 +1588,7 @@ edb_status launch_calq32_batch(int N, int S, const float *d_B32, const float2 *d
     C32MultiIn one{N, S, d_B32, d_fin, d_Q};
     one.C = C;
     one.partial = d_partial;
-    EDB_TRY(launch_calq32_multi(1, &one, variant, st, persist < 0));
+    EDB_TRY(launch_calq32_multi(1, &one, variant, st, persist < 0 && C == 1));
     if (C == 1) return EDB_OK;
     return launch_c32_reduce(N, S, C, d_partial, d_Q, st);
   }
@@ -1583,7 +1613,7 @@ template <int V>
 static edb_status launch_c32_multi_v(const C32Multi &mt, int block, size_t smem,
                                      cudaStream_t st) {
   constexpr C32Variant vr = kC32Variants[V];
-  auto kern = calq32_multi_kernel<true, vr.maxt, vr.hls, vr.ws, vr.a, vr.minb, false>;
+  auto kern = calq32_multi_kernel<true, vr.maxt, vr.hls, vr.ws, vr.a, vr.minb, false, vr.sc>;
   static const cudaError_t configured = cudaFuncSetAttribute(
       kern, cudaFuncAttributeMaxDynamicSharedMemorySize, vr.minb == 2 ? 113 * 1024 : 227 * 1024);
   if (configured != cudaSuccess) return cuda_fail(configured, "cudaFuncSetAttribute(calq32 multi)");
@@ -1624,7 +1654,7 @@ edb_status launch_calq32_multi(int ntab, const C32MultiIn *in, int variant, cuda
   if (variant < 0 || variant >= calq32_variants() || kC32Variants[variant].pair)
     return fail(EDB_EINVAL, "calq32 multi: a plain-layout variant (0-4)");
   const C32Variant &vr = kC32Variants[variant];
-  const int SG = SC * vr.ws;
+  const int SG = vr.sc * vr.ws;
   std::vector<int> order(ntab);
   for (int i = 0; i < ntab; ++i) order[i] = i;
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return in[a].N > in[b].N; });
@@ -1688,6 +1718,8 @@ edb_status launch_calq32_multi(int ntab, const C32MultiIn *in, int variant, cuda
     case 1: rc = launch_c32_multi_v<1>(mt, block, smem, st); break;
     case 2: rc = launch_c32_multi_v<2>(mt, block, smem, st); break;
     case 3: rc = launch_c32_multi_v<3>(mt, block, smem, st); break;
+    case 10: rc = launch_c32_multi_v<10>(mt, block, smem, st); break;
+    case 11: rc = launch_c32_multi_v<11>(mt, block, smem, st); break;
     default: rc = launch_c32_multi_v<4>(mt, block, smem, st); break;
   }
   const cudaError_t fe = queue ? cudaFreeAsync(mt.queue, st) : cudaSuccess;
