@@ -255,7 +255,7 @@ constexpr int MAX_ST = 4;                 // pipeline stages (l-lines in flight)
 static_assert((2 * MAX_ST + 2) * 8 + MAX_ST * 4 <= 120, "shared-memory header");
 
 struct C32Geom {
-  int N, A, R, RA, K2T, BROW, FLS, PSTR, NST, NPL, HLT, SG, EL;
+  int N, A, R, RA, K2T, BROW, FLS, PSTR, NST, NPL, HLT, SG, EL, LPS;
   int BSTG, FSTG;  // per-stage sizes: B tile (floats), f_l lines (float2)
   size_t off_B, off_fl, off_pl, off_hl, bytes;
 };
@@ -268,9 +268,12 @@ struct C32Geom {
 // each stage's last fill).  SG data units (solves, or
 // solve pairs) of EL float2 per element (1: (re, im); 2: (re_a, re_b),
 // (im_a, im_b) of a pair).
+// LPS l-lines share a stage (and its barriers): [line] tiles of B, [unit][line]
+// f_l lines.
 __host__ __device__ inline C32Geom c32_geom(int N, int A, int K2T, int NST, int NPL, int HLT,
-                                            int SG, int EL, bool TMA) {
+                                            int SG, int EL, bool TMA, int LPS = 1) {
   C32Geom g;
+  g.LPS = LPS;
   g.SG = SG;
   g.EL = EL;
   g.A = A;
@@ -294,8 +297,8 @@ __host__ __device__ inline C32Geom c32_geom(int N, int A, int K2T, int NST, int 
     g.PSTR = (N * N + (9 - (N * N) % 8) % 8) * EL;
   }
   size_t o = 128;  // 2*MAX_ST + 2 mbarriers, MAX_ST fill counts (+ pad)
-  g.BSTG = g.RA * g.BROW;
-  g.FSTG = SG * g.FLS;
+  g.BSTG = LPS * g.RA * g.BROW;
+  g.FSTG = SG * LPS * g.FLS;
   if (TMA) {
     g.BSTG = (g.BSTG + 31) / 32 * 32;
     g.FSTG = (g.FSTG + 15) / 16 * 16;
@@ -501,7 +504,7 @@ __device__ __forceinline__ void stage_line(const C32Geom &g, int li, int vl, int
   const int rowlen = k2n * N;
   if (TMA && tmap) {  // called by the issuing warp only
     if ((threadIdx.x & 31) == 0) {
-      mbar_expect_tx(full + st, (uint32_t)(N * g.K2T * N * 4 + g.SG * g.FLS * 8));
+      mbar_expect_tx(full + st, (uint32_t)(g.LPS * (N * g.K2T * N * 4 + g.SG * g.FLS * 8)));
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       tma_load_5d(Bd, tmB, 0, k2_0, 0, vl, k1, full + st);
       tma_load_3d(fd, tmF, 0, li, s0, full + st);
@@ -747,7 +750,13 @@ __device__ __forceinline__ void compute_line_al(const C32Geom &g, const float *B
 #pragma unroll(RC > 0 ? RC : 1)
   for (int gg = 0; gg < (RC > 0 ? RC : g.R); ++gg) {
     const int qq = base == 0 ? N : base;
+    uint32_t qa[SN];
     ulonglong2 fp[SN];  // f_l of steps (t, t + 1)
+#pragma unroll
+    for (int c = 0; c < SN; ++c) {
+      qa[c] = sp[c] + 8u * qq;
+      fp[c] = make_ulonglong2(0ull, 0ull);
+    }
 #pragma unroll
     for (int t = 0; t < A; ++t) {
       // the ring entry of step t: f_m at qq - t (t = 0: base, held over)
@@ -758,7 +767,7 @@ __device__ __forceinline__ void compute_line_al(const C32Geom &g, const float *B
       } else if (t & 1) {  // pair (qq - t - 1, qq - t)
 #pragma unroll
         for (int c = 0; c < SN; ++c) {
-          const ulonglong2 v = lds_u64x2(sp[c] + 8u * qq - 8u * (t + 1));
+          const ulonglong2 v = lds_u64x2(qa[c] - 8u * (t + 1));
           ring[(A - t) % A][c] = v.y;
           held[c] = v.x;
         }
@@ -922,13 +931,15 @@ __device__ __forceinline__ bool calq32_cta(int N, int S, int K2T, int NST, int N
                                            float2 *__restrict__ Q, float4 *__restrict__ partial,
                                            int tmap, unsigned long long wait_ns,
                                            const CUtensorMap *tmB, const CUtensorMap *tmF, int U,
-                                           int GY, int GZ, long long lin, int nthr) {
+                                           int GY, int GZ, long long lin, int nthr, int lps) {
   constexpr int SC = SN;       // solves per thread: w and, with two, w + WS
+  // lines of a stage (N % 4 == 0 and lps divides 4 where it is not 1)
+  const int LPS = SN == 1 ? lps : 1;
   constexpr int SG = SC * WS;  // solves per group
   extern __shared__ __align__(128) unsigned char smem[];
   const C32Geom g =
       c32_geom(N, A, K2T, NST, NPL, HLS ? (int)blockDim.x : 0, PAIR ? WS : SG, PAIR ? 2 : 1,
-               TMA && tmap);
+               TMA && tmap, LPS);
   uint64_t *full = reinterpret_cast<uint64_t *>(smem);  // [MAX_ST]
   uint64_t *empty = full + MAX_ST;                       // [MAX_ST]
   uint64_t *pbar = full + 2 * MAX_ST;                    // [2] planes
@@ -980,7 +991,7 @@ __device__ __forceinline__ bool calq32_cta(int N, int S, int K2T, int NST, int N
   const int PPC = (nlist + C - 1) / C;
   const int P0 = min(nlist, chunk * PPC), P1 = min(nlist, P0 + PPC);
   const int nplanes = P1 - P0;
-  const int nlines = nplanes * N;
+  const int nlines = nplanes * N / LPS;  // stages of LPS lines
   auto line_li = [&](int j) { return plane_l1(P0 + j / N) * N + j % N; };
   const size_t plane_sz = (size_t)g.SG * g.PSTR;
   const bool ring_al = (N % A) == 0;  // compute_line*_al apply (tensor-copy path)
@@ -1030,7 +1041,7 @@ __device__ __forceinline__ bool calq32_cta(int N, int S, int K2T, int NST, int N
   int planes = 0;       // counted in warp 0
   if (TMA && warp == 0 && nlines > 0) {
     for (int j = 0; j < NST - 1 && j < nlines; ++j) {
-      stage_line<true>(g, line_li(j), P0 * N + j, j % NST, k1, k2_0, k2n, u0, nval, NQ, B32, fin, Bs, fls,
+      stage_line<true>(g, line_li(j * LPS), P0 * N + j * LPS, j % NST, k1, k2_0, k2n, u0, nval, NQ, B32, fin, Bs, fls,
                        full, tmap, tmB, tmF);
       if (lane == 0) ++fills[j % NST];
     }
@@ -1087,13 +1098,18 @@ __device__ __forceinline__ bool calq32_cta(int N, int S, int K2T, int NST, int N
         const int sn = st == 0 ? NST - 1 : st - 1;
         if (j >= 1) mbar_wait(&empty[sn], (uint32_t)(st > 0 ? fpar : fpar ^ 1), to, wait_ns);
         if (!__any_sync(warp_mask(), to)) {
-          // line jn is row l2 + NST - 1 of plane pr, or of plane pr + 1 (NST <= N)
-          int l2n = l2 + NST - 1, prn = pr;
-          if (l2n >= N) {
+          // its first line is row l2 + (NST - 1) LPS of plane pr, or of a later one
+          int l2n = l2 + (NST - 1) * LPS, prn = pr;
+          if constexpr (SN == 1) {
+            while (l2n >= N) {
+              l2n -= N;
+              ++prn;
+            }
+          } else if (l2n >= N) {  // NST <= N
             l2n -= N;
             ++prn;
           }
-          stage_line<true>(g, plane_l1(P0 + prn) * N + l2n, P0 * N + jn, sn, k1, k2_0, k2n, u0,
+          stage_line<true>(g, plane_l1(P0 + prn) * N + l2n, P0 * N + jn * LPS, sn, k1, k2_0, k2n, u0,
                            nval, NQ, B32, fin, Bs, fls, full, tmap, tmB, tmF);
           if (lane == 0) ++fills[sn];
         }
@@ -1108,32 +1124,41 @@ __device__ __forceinline__ bool calq32_cta(int N, int S, int K2T, int NST, int N
 
     // ---- compute line (l1, l2)
     if (act) {
-    const float *Bt = Bs + (size_t)st * g.BSTG + k2l * N + k3_0;
-    const float2 *fl0 = fls + (size_t)st * g.FSTG + (size_t)w * g.FLS;
-    const float2 *p0 = plb + (size_t)pb * plane_sz + (size_t)w * g.PSTR + m2 * N * g.EL;
-    const float2 *fl1 = fl0 + (size_t)WS * g.FLS;
-    const float2 *p1 = p0 + (size_t)WS * g.PSTR;
-    if constexpr (SC == 1) {  // tensor-copy path with N % A == 0 only (see the launcher)
-      compute_line_al_n<A, 1>(g, Bt, fl0, fl1, p0, p1, k3_0, accA, accB);
-    } else if constexpr (PAIR) {
-      if (TMA && ring_al && FIXN)
-        compute_line_pair_al_n<A>(g, Bt, fl0, p0, k3_0, accA, accB);
-      else if (TMA && ring_al)
-        compute_line_pair_al<A>(g, Bt, fl0, p0, k3_0, accA, accB);
-      else if (TMA)
-        compute_line_pair<true, true, A>(g, Bt, fl0, p0, k3_0, accA, accB);
-      else
-        compute_line_pair<false, false, A>(g, Bt, fl0, p0, k3_0, accA, accB);
-    } else {
-      if (TMA && ring_al && FIXN)
-        compute_line_al_n<A, 2>(g, Bt, fl0, fl1, p0, p1, k3_0, accA, accB);
-      else if (TMA && ring_al)
-        compute_line_al<A, 0, 2>(g, Bt, fl0, fl1, p0, p1, k3_0, accA, accB);
-      else if (TMA)
-        compute_line<true, true, A>(g, Bt, fl0, fl1, p0, p1, k3_0, accA, accB);
-      else
-        compute_line<false, false, A>(g, Bt, fl0, fl1, p0, p1, k3_0, accA, accB);
-    }
+      const float *Bt = Bs + (size_t)st * g.BSTG + k2l * N + k3_0;
+      const float2 *fl0 = fls + (size_t)st * g.FSTG + (size_t)w * g.FLS;
+      const float2 *p0 = plb + (size_t)pb * plane_sz + (size_t)w * g.PSTR + m2 * N * g.EL;
+      const float2 *fl1 = fl0 + (size_t)WS * g.FLS;
+      const float2 *p1 = p0 + (size_t)WS * g.PSTR;
+      if constexpr (SC == 1) {  // tensor-copy path with N % A == 0 only (see the launcher)
+        fl0 = fls + (size_t)st * g.FSTG + (size_t)(w * LPS) * g.FLS;
+        int m2s = m2;
+#pragma unroll 1
+        for (int sub = 0; sub < LPS; ++sub) {
+          p0 = plb + (size_t)pb * plane_sz + (size_t)w * g.PSTR + m2s * N;
+          compute_line_al_n<A, 1>(g, Bt, fl0, fl1, p0, p1, k3_0, accA, accB);
+          Bt += g.RA * g.BROW;
+          fl0 += g.FLS;
+          m2s = m2s == 0 ? N - 1 : m2s - 1;
+        }
+      } else if constexpr (PAIR) {
+        if (TMA && ring_al && FIXN)
+          compute_line_pair_al_n<A>(g, Bt, fl0, p0, k3_0, accA, accB);
+        else if (TMA && ring_al)
+          compute_line_pair_al<A>(g, Bt, fl0, p0, k3_0, accA, accB);
+        else if (TMA)
+          compute_line_pair<true, true, A>(g, Bt, fl0, p0, k3_0, accA, accB);
+        else
+          compute_line_pair<false, false, A>(g, Bt, fl0, p0, k3_0, accA, accB);
+      } else {
+        if (TMA && ring_al && FIXN)
+          compute_line_al_n<A, 2>(g, Bt, fl0, fl1, p0, p1, k3_0, accA, accB);
+        else if (TMA && ring_al)
+          compute_line_al<A, 0, 2>(g, Bt, fl0, fl1, p0, p1, k3_0, accA, accB);
+        else if (TMA)
+          compute_line<true, true, A>(g, Bt, fl0, fl1, p0, p1, k3_0, accA, accB);
+        else
+          compute_line<false, false, A>(g, Bt, fl0, fl1, p0, p1, k3_0, accA, accB);
+      }
     }
     if (TMA) {
       // a warp releases the stage only when every lane saw this line's copy
@@ -1142,7 +1167,7 @@ __device__ __forceinline__ bool calq32_cta(int N, int S, int K2T, int NST, int N
       const bool bad = __any_sync(warp_mask(), to);
       if (lane == 0 && !bad) mbar_arrive(&empty[st]);
     }
-    if ((l2 + 1) % FOLD_LINES == 0 || l2 == N - 1) {  // fold into the compensated pair
+    if ((l2 + LPS) % FOLD_LINES == 0 || l2 == N - LPS) {  // fold into the compensated pair
 #pragma unroll
       for (int a = 0; a < A; ++a) {
         // (accA.x - accB.y, accA.y + accB.x) = accA + (-1, 1) * swap(accB);
@@ -1177,12 +1202,12 @@ __device__ __forceinline__ bool calq32_cta(int N, int S, int K2T, int NST, int N
       st = 0;
       fpar ^= 1;
     }
-    if (++l2 == N) {
+    if ((l2 += LPS) == N) {
       l2 = 0;
       m2 = k2c;
       if (++pr < nplanes) l1 = plane_l1(P0 + pr);
     } else {
-      m2 = m2 == 0 ? N - 1 : m2 - 1;
+      m2 = m2 >= LPS ? m2 - LPS : m2 - LPS + N;
     }
     if (++iw == nfull) iw = 0;
   }
@@ -1270,7 +1295,7 @@ __global__ void __launch_bounds__(MAXT, MINB)
       blockIdx.x + (long long)gridDim.x * (blockIdx.y + (long long)gridDim.y * blockIdx.z);
   calq32_cta<TMA, MAXT, HLS, WS, A, MINB, PAIR, 2>(N, S, K2T, NST, NPL, C, GB, B32, fin, Q, partial,
                                                tmap, wait_ns, &tmB, &tmF, gridDim.x, gridDim.y,
-                                               gridDim.z, lin, (int)blockDim.x);
+                                               gridDim.z, lin, (int)blockDim.x, 1);
 }
 
 // Several tables in one persistent launch (uneven N, each table shared by its
@@ -1287,7 +1312,7 @@ struct C32Table {
   float2 *Q;
   long long begin;
   float4 *partial;  // C > 1: chunk partial sums
-  int N, S, K2T, NST, NPL, GB, U, GY, GZ, tmap, threads, C;
+  int N, S, K2T, NST, NPL, GB, U, GY, GZ, tmap, threads, C, LPS;
 };
 constexpr int C32_MULTI_MAX = 16;
 struct C32Multi {
@@ -1320,7 +1345,7 @@ __global__ void __launch_bounds__(MAXT, MINB)
     const C32Table &d = mt.t[t];
     const bool ok = calq32_cta<TMA, MAXT, HLS, WS, A, MINB, PAIR, SN>(
         d.N, d.S, d.K2T, d.NST, d.NPL, d.C, d.GB, d.B32, d.fin, d.Q, d.partial, d.tmap, wait_ns,
-        &d.tmB, &d.tmF, d.U, d.GY, d.GZ, item - d.begin, d.threads);
+        &d.tmB, &d.tmF, d.U, d.GY, d.GZ, item - d.begin, d.threads, d.LPS);
     if (!ok) break;  // uniform: the CTA drained its copies and set the status word
     // every thread is done with the item; the barriers (at the start of shared
     // memory) are invalidated before the next item initialises them again
@@ -1361,21 +1386,26 @@ __global__ void calq32_reduce_kernel(long long n, int C, const float4 *__restric
 //        shared-memory loads; needs a pair-layout copy of the input)
 //   10: WS 4, A 4, one solve a thread (4-solve groups), <= 256 threads
 //   11: WS 2, the same (2-solve groups)
-// 10 and 11 are for the few solves that leave 16-solve lanes empty: TIMING_S
+//   12, 13: 10 and 11 with stages kept small enough for one wave of CTAs
+// 10-13 are for the few solves that leave 16-solve lanes empty.  us without
+// chunks, best of 0-9 -> best of 10-13: 4 x N = 16 191 -> 95, 4 x N = 24 718 -> 244,
+// 4 x N = 32 2100 -> 1000; in 4 chunks 76 -> 49, 296 -> 224, 2126 -> 760.
 struct C32Variant {
   int ws, a, maxt;
   bool hls;
   int minb;
   bool pair;
   int sc;  // solves per thread
+  bool wave;  // one-solve variants: stages no deeper than one wave of CTAs allows
 };
 constexpr C32Variant kC32Variants[] = {
-    {8, 8, 256, false, 1, false, 2}, {8, 8, 384, true, 1, false, 2},
-    {2, 8, 256, false, 1, false, 2}, {8, 4, 256, false, 2, false, 2},
-    {8, 4, 384, false, 1, false, 2}, {8, 8, 256, false, 1, true, 2},
-    {8, 8, 384, true, 1, true, 2},   {2, 8, 256, false, 1, true, 2},
-    {8, 4, 256, false, 2, true, 2},  {8, 4, 384, false, 1, true, 2},
-    {4, 4, 256, false, 2, false, 1}, {2, 4, 256, false, 2, false, 1}};
+    {8, 8, 256, false, 1, false, 2, false}, {8, 8, 384, true, 1, false, 2, false},
+    {2, 8, 256, false, 1, false, 2, false}, {8, 4, 256, false, 2, false, 2, false},
+    {8, 4, 384, false, 1, false, 2, false}, {8, 8, 256, false, 1, true, 2, false},
+    {8, 8, 384, true, 1, true, 2, false},   {2, 8, 256, false, 1, true, 2, false},
+    {8, 4, 256, false, 2, true, 2, false},  {8, 4, 384, false, 1, true, 2, false},
+    {4, 4, 256, false, 2, false, 1, false}, {2, 4, 256, false, 2, false, 1, false},
+    {4, 4, 256, false, 2, false, 1, true},  {2, 4, 256, false, 2, false, 1, true}};
 int calq32_variants() { return (int)(sizeof(kC32Variants) / sizeof(kC32Variants[0])); }
 int calq32_group(int variant) { return kC32Variants[variant].sc * kC32Variants[variant].ws; }
 bool calq32_pair(int variant) { return kC32Variants[variant].pair; }
@@ -1461,7 +1491,7 @@ static edb_status launch_c32_variant(int v, dim3 grid, int threads, size_t smem,
 // launch (the same for a single-table and a grouped launch).  src: the input
 // the f_l lines and planes are staged from (the solve-pair copy for PAIR).
 struct C32Setup {
-  int K2T, tiles, threads, NST, NPL, GB;
+  int K2T, tiles, threads, NST, NPL, GB, LPS;
   bool tma;
   C32Maps maps;
   size_t bytes;
@@ -1495,8 +1525,46 @@ static edb_status c32_setup(int N, int S, const C32Variant &vr, int C, const flo
   // line staging by two tensor copies when the f_l box fits (<= 256 floats a
   // row), else by one bulk copy per B row and f_l line
   o->maps = C32Maps{};
-  if (o->tma && 2 * c32_geom(N, A, K2T, 1, 1, 0, units, el, true).FLS <= 256 && N <= 256) {
-    const int FLS = c32_geom(N, A, K2T, 1, 1, 0, units, el, true).FLS;
+  const int FLS = c32_geom(N, A, K2T, 1, 1, 0, units, el, true).FLS;
+  const bool boxes = o->tma && 2 * FLS <= 256 && N <= 256;
+  // deepest pipeline that fits: two planes with >= 3 stages if possible,
+  // else one plane with up to MAX_ST stages (the plain path uses 1 + 1).
+  const size_t cap = vr.minb == 2 ? 113 * 1024 : 227 * 1024;
+  int NST = 1, NPL = 1, lps = 1;
+  if (o->tma) {
+    NST = 0;
+    auto find = [&](int l, int ns_min, int npl) {
+      for (int ns = MAX_ST; ns >= ns_min && !NST; --ns)
+        if (c32_geom(N, A, K2T, ns, npl, hlt, units, el, boxes, l).bytes <= cap) {
+          NST = ns;
+          NPL = npl;
+        }
+    };
+    // The one-solve variants stage up to a fold's four lines together: their
+    // tiles are small, and a line's barriers cost more than its sums (4 x N = 16:
+    // 142 us with one line a stage, 95 with four), but not where that leaves a
+    // CTA fewer than 24 stages to walk.  Whether more CTAs than fit on the SMs at
+    // once are worth it depends on the size (16 x N = 16: 102 us in one wave, 177
+    // with deep stages in two; 8 x N = 24: 697 and 475), so both are variants.
+    const long long ctas = (long long)((S + SG - 1) / SG) * C * N * tiles;
+    const int lines = (c32_maxlist(N) + C - 1) / C * N;
+    if (vr.sc == 1 && boxes)
+      for (int l = FOLD_LINES; l > 1 && !NST; l /= 2) {
+        if (lines / l < 24) continue;
+        for (int npl = 2; npl >= 1 && !NST; --npl) {
+          find(l, 3, npl);
+          if (!NST) continue;
+          const size_t b = c32_geom(N, A, K2T, NST, NPL, hlt, units, el, boxes, l).bytes + 1024;
+          if (vr.wave && ctas > (long long)device_sm_count() * (long long)(228 * 1024 / b)) NST = 0;
+        }
+        lps = NST ? l : 1;
+      }
+    if (!NST) find(1, 3, 2);
+    if (!NST) find(1, 2, 1);
+    if (!NST) return fail(EDB_EINVAL, "calq32: this variant does not fit in shared memory");
+  }
+  o->LPS = lps;
+  if (boxes) {
     const long long NQ = (long long)N * N * N;
     // pair table [k1][visited line][l3][k2][k3]: dims k3, k2, l3, visited line, k1
     const long long VL = (long long)c32_maxlist(N) * N;
@@ -1504,34 +1572,16 @@ static edb_status c32_setup(int N, int S, const C32Variant &vr, int C, const flo
                                 (cuuint64_t)N};
     const cuuint64_t bstr[4] = {(cuuint64_t)N * 4, (cuuint64_t)N * N * 4, (cuuint64_t)NQ * 4,
                                 (cuuint64_t)(VL * NQ * 4)};
-    const cuuint32_t bbox[5] = {(cuuint32_t)N, (cuuint32_t)K2T, (cuuint32_t)N, 1, 1};
+    const cuuint32_t bbox[5] = {(cuuint32_t)N, (cuuint32_t)K2T, (cuuint32_t)N, (cuuint32_t)lps, 1};
     const long long nunits = vr.pair ? (S + 1) / 2 : S;
     const cuuint64_t fdim[3] = {(cuuint64_t)N * 2 * el, (cuuint64_t)N * N, (cuuint64_t)nunits};
     const cuuint64_t fstr[2] = {(cuuint64_t)N * 8 * el, (cuuint64_t)NQ * 8 * el};
-    const cuuint32_t fbox[3] = {(cuuint32_t)(2 * FLS), 1, (cuuint32_t)units};
+    const cuuint32_t fbox[3] = {(cuuint32_t)(2 * FLS), (cuuint32_t)lps, (cuuint32_t)units};
     if (encode_map(&o->maps.B, 5, d_B32, bdim, bstr, bbox) &&
         encode_map(&o->maps.F, 3, src, fdim, fstr, fbox))
       o->maps.tmap = 1;
   }
-  // deepest pipeline that fits: two planes with >= 3 stages if possible,
-  // else one plane with up to MAX_ST stages (the plain path uses 1 + 1)
-  const size_t cap = vr.minb == 2 ? 113 * 1024 : 227 * 1024;
-  int NST = 1, NPL = 1;
-  if (o->tma) {
-    NST = 0;
-    for (int ns = MAX_ST; ns >= 3 && !NST; --ns)
-      if (c32_geom(N, A, K2T, ns, 2, hlt, units, el, o->maps.tmap).bytes <= cap) {
-        NST = ns;
-        NPL = 2;
-      }
-    for (int ns = MAX_ST; ns >= 2 && !NST; --ns)
-      if (c32_geom(N, A, K2T, ns, 1, hlt, units, el, o->maps.tmap).bytes <= cap) {
-        NST = ns;
-        NPL = 1;
-      }
-    if (!NST) return fail(EDB_EINVAL, "calq32: this variant does not fit in shared memory");
-  }
-  const C32Geom g = c32_geom(N, A, K2T, NST, NPL, hlt, units, el, o->maps.tmap);
+  const C32Geom g = c32_geom(N, A, K2T, NST, NPL, hlt, units, el, o->maps.tmap, lps);
   if (g.bytes > cap) return fail(EDB_EINVAL, "calq32: this variant does not fit in shared memory");
   o->NST = NST;
   o->NPL = NPL;
@@ -1609,8 +1659,15 @@ edb_status launch_calq32_batch(int N, int S, const float *d_B32, const float2 *d
   return launch_c32_reduce(N, S, C, d_partial, d_Q, st);
 }
 
+// The work queue's counter, stream-ordered: allocated, zeroed, used, freed.
+static edb_status queue_alloc(unsigned long long **p, cudaStream_t st) {
+  EDB_CUDA(cudaMallocAsync(reinterpret_cast<void **>(p), sizeof(**p), st));
+  EDB_CUDA(cudaMemsetAsync(*p, 0, sizeof(**p), st));
+  return EDB_OK;
+}
+
 template <int V>
-static edb_status launch_c32_multi_v(const C32Multi &mt, int block, size_t smem,
+static edb_status launch_c32_multi_v(C32Multi &mt, int block, size_t smem, bool queue,
                                      cudaStream_t st) {
   constexpr C32Variant vr = kC32Variants[V];
   auto kern = calq32_multi_kernel<true, vr.maxt, vr.hls, vr.ws, vr.a, vr.minb, false, vr.sc>;
@@ -1638,8 +1695,15 @@ static edb_status launch_c32_multi_v(const C32Multi &mt, int block, size_t smem,
   }
   if (occ < 1) return fail(EDB_EINVAL, "calq32 multi: the block does not fit on an SM");
   const long long blocks = std::min<long long>(mt.total, (long long)occ * device_sm_count());
+  // a grid that holds every item at once needs no queue
+  mt.queue = nullptr;
+  if (queue && mt.total > blocks) EDB_TRY(queue_alloc(&mt.queue, st));
   kern<<<(unsigned)blocks, block, smem, st>>>(mt, wait_limit_ns());
-  EDB_LAUNCHED();
+  count_launch();
+  const cudaError_t le = cudaGetLastError();
+  const cudaError_t fe = mt.queue ? cudaFreeAsync(mt.queue, st) : cudaSuccess;
+  if (le != cudaSuccess) return cuda_fail(le, "kernel launch");
+  if (fe != cudaSuccess) return cuda_fail(fe, "cudaFreeAsync(calq32 multi queue)");
   return EDB_OK;
 }
 
@@ -1694,6 +1758,7 @@ edb_status launch_calq32_multi(int ntab, const C32MultiIn *in, int variant, cuda
     d.NST = su.NST;
     d.NPL = su.NPL;
     d.GB = su.GB;
+    d.LPS = su.LPS;
     d.U = (e.S + SG - 1) / SG * e.C;
     d.C = e.C;
     d.partial = e.partial;
@@ -1705,27 +1770,17 @@ edb_status launch_calq32_multi(int ntab, const C32MultiIn *in, int variant, cuda
     smem = std::max(smem, su.bytes);
   }
   mt.total = begin;
-  // the work queue's counter, stream-ordered: allocated, zeroed, used, freed
-  mt.queue = nullptr;
-  if (queue) {
-    EDB_CUDA(
-        cudaMallocAsync(reinterpret_cast<void **>(&mt.queue), sizeof(unsigned long long), st));
-    EDB_CUDA(cudaMemsetAsync(mt.queue, 0, sizeof(unsigned long long), st));
-  }
-  edb_status rc;
   switch (variant) {
-    case 0: rc = launch_c32_multi_v<0>(mt, block, smem, st); break;
-    case 1: rc = launch_c32_multi_v<1>(mt, block, smem, st); break;
-    case 2: rc = launch_c32_multi_v<2>(mt, block, smem, st); break;
-    case 3: rc = launch_c32_multi_v<3>(mt, block, smem, st); break;
-    case 10: rc = launch_c32_multi_v<10>(mt, block, smem, st); break;
-    case 11: rc = launch_c32_multi_v<11>(mt, block, smem, st); break;
-    default: rc = launch_c32_multi_v<4>(mt, block, smem, st); break;
+    case 0: return launch_c32_multi_v<0>(mt, block, smem, queue, st);
+    case 1: return launch_c32_multi_v<1>(mt, block, smem, queue, st);
+    case 2: return launch_c32_multi_v<2>(mt, block, smem, queue, st);
+    case 3: return launch_c32_multi_v<3>(mt, block, smem, queue, st);
+    case 10:
+    case 12: return launch_c32_multi_v<10>(mt, block, smem, queue, st);
+    case 11:
+    case 13: return launch_c32_multi_v<11>(mt, block, smem, queue, st);
+    default: return launch_c32_multi_v<4>(mt, block, smem, queue, st);
   }
-  const cudaError_t fe = queue ? cudaFreeAsync(mt.queue, st) : cudaSuccess;
-  if (rc != EDB_OK) return rc;
-  if (fe != cudaSuccess) return cuda_fail(fe, "cudaFreeAsync(calq32 multi queue)");
-  return EDB_OK;
 }
 
 edb_status calq32_status_ptr(int **p) {

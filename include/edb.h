@@ -153,7 +153,8 @@ edb_status edb_qcalc_calQ_batch_f32_device(edb_qcalc *q, int S, const float *d_f
  * threads with the compensated sums in registers / <= 384 threads with them
  * in shared memory); 2: 4-solve groups; 3/4: 4 outputs per thread (2 CTAs
  * per SM / 384 threads).  Variants 5-9 are 0-4 on a solve-pair copy of the
- * input, kept by the handle.  chunks > 1 splits the l1 planes into that many
+ * input, kept by the handle.  10-13: one solve a thread, for few solves (10, 12:
+ * 4-solve groups; 11, 13: 2-solve groups; 12, 13 with smaller stages).  chunks > 1 splits the l1 planes into that many
  * chunks whose compensated sums are added in order in FP64; d_partial
  * (device) then holds chunks x S x N^3 x 16 bytes.  For a given chunk count
  * the result of each solve does not depend on S or the variant.  Without
