@@ -1,6 +1,7 @@
 // Internal declarations shared by the libedb translation units.
 #pragma once
 
+#include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -127,6 +128,10 @@ edb_status launch_calq64_reduce(const QParams &p, int nchunk, const double2 *d_p
 // {re_hi, im_hi, re_lo, im_lo}.
 // d_partial holds calq64x_nchunk(p) * KC.
 int calq64x_nchunk(const QParams &p, int *J2T_out);
+// FP32 tiled tensor map, no swizzle, out-of-bounds elements read as zero;
+// false: the driver has no encoder or refused the map.
+bool encode_map(CUtensorMap *m, int rank, const void *base, const cuuint64_t *dim,
+                const cuuint64_t *stride, const cuuint32_t *box);
 edb_status launch_split_f(long long n, const double2 *f, float4 *out, cudaStream_t st);
 edb_status launch_split_B(long long n, const double *B, float2 *B2, cudaStream_t st);
 // ALIASED tables: B2 = split of the symmetric pair table (B[l][k] + B[k-l][k]

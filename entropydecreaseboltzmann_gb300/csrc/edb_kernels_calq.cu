@@ -1436,8 +1436,8 @@ static EncodeTiledFn encode_tiled() {
   return fn;
 }
 // FP32 tiled map, no swizzle, out-of-bounds elements read as zero.
-static bool encode_map(CUtensorMap *m, int rank, const void *base, const cuuint64_t *dim,
-                       const cuuint64_t *stride, const cuuint32_t *box) {
+bool encode_map(CUtensorMap *m, int rank, const void *base, const cuuint64_t *dim,
+                const cuuint64_t *stride, const cuuint32_t *box) {
   const EncodeTiledFn fn = encode_tiled();
   if (!fn) return false;
   const cuuint32_t es[5] = {1, 1, 1, 1, 1};

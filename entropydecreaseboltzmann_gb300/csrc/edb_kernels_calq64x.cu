@@ -41,10 +41,12 @@
 //
 // B stream: when every warp's row segment is a contiguous, 16-byte aligned run
 // (P % 4 == 0 and whole j2 tiles), each warp streams its own 1 KB segment of
-// the next D rows into a private shared-memory ring with 1-D TMA bulk copies
-// (lane 0 issues; one mbarrier per slot; waits bounded by %globaltimer, a
-// timeout sets the device status word).  Otherwise threads load their 32
+// the next D rows into a private shared-memory ring with TMA copies (1-D bulk
+// copies here, boxes of rows in calq64p_kernel; lane 0 issues; one mbarrier per
+// slot; waits bounded by %globaltimer, a timeout sets the device status word).  Otherwise threads load their 32
 // bytes per row with __ldg, one row ahead.
+#include <cuda.h>
+
 #include <algorithm>
 #include <functional>
 #include <map>
@@ -132,6 +134,21 @@ __device__ __forceinline__ void mbar_wait_nz(uint64_t *bar, uint32_t parity, boo
       return;
     }
   }
+}
+
+// A slot's refill from the lanes with `on`, by predication (a divergent block for
+// one lane costs its warp about 70 clocks beside its instructions): the bytes the
+// barrier waits for, and one tensor copy of the box of rows at (x, row).
+__device__ __forceinline__ void box_g2s(uint32_t dst, const CUtensorMap *tm, int x, int row,
+                                        uint32_t bytes, uint32_t bar, bool on) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.b32 p, %6, 0;\n"
+      " @p fence.proxy.async.shared::cta;\n"
+      " @p mbarrier.arrive.expect_tx.shared::cta.b64 _, [%4], %5;\n"
+      " @p cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%2, %3}], [%4];\n}\n" ::"r"(dst),
+      "l"(reinterpret_cast<uint64_t>(tm)), "r"(x), "r"(row), "r"(bar), "r"(bytes), "r"((int)on)
+      : "memory");
 }
 
 __device__ int g_calq64x_status;  // nonzero: a bounded wait ran out
@@ -481,14 +498,15 @@ __global__ void __launch_bounds__(MAXT, MINB)
 // (x mod 4) N/4 + x/4: the lanes of a row read x four apart, which then fall
 // in distinct 16-byte bank groups (at N = 32 every 128-bit load is
 // conflict-free; untransposed, eight lanes shared one group).
-// B stream: ROWS table rows per ring slot (one wait, one vote and one
-// expect_tx per slot), PDEPTH rows in flight per warp.
+// B stream: ROWS table rows per ring slot (one wait, one vote and one tensor
+// copy per slot), PDEPTH rows in flight per warp.  The kernel is bound by the
+// issue of its double-float arithmetic (57 packed instructions for two outputs
+// and one table row), so what a refill adds to a warp counts: one bulk copy per
+// row from a block that only lane 0 entered took 6 to 23% of the time (N = 16
+// 51 -> 40 us, 20 125 -> 105, 24 286 -> 262, 28 704 -> 605, 32 1125 -> 1053),
+// against one copy of all ROWS rows, issued by predication, whose row number
+// every lane carries.
 constexpr int PDEPTH = 8;
-struct __align__(16) P64Cursor {
-  const float4 *src;
-  int pi, i2, i3;
-  int issued;  // slot fills the warp has issued
-};
 
 // fdr: f-hat split as for calq64x_kernel and rotated along the last axis by
 // the f_l shift, fdr[a1][a2][i] = f[a1][a2][(i + sL) mod N], with one float4 of
@@ -496,11 +514,14 @@ struct __align__(16) P64Cursor {
 // read one step ahead touches entry N, the next row's first or the padding).
 // An f_m entry x (FFTW order) sits at (x + n) mod N of its row.
 // NC > 0: N fixed at compile time (the index arithmetic folds); 0: p.N.
+// tmB: the table as N^3 rows of 2 N^3 floats, box ROWS rows of a full warp's
+// segment (the last warp, where it is short, copies a full box too: the columns
+// past its own are other threads' and are not read).
 template <bool TMA, int MAXT, int MINB, int ROWS, int NC>
 __global__ void __launch_bounds__(MAXT, MINB)
     calq64p_kernel(QParams p, int J2T, int LC, const float4 *__restrict__ B2p,
                    const float4 *__restrict__ fdr, double2 *__restrict__ partial,
-                   unsigned long long wait_ns) {
+                   unsigned long long wait_ns, const __grid_constant__ CUtensorMap tmB) {
   constexpr int SLOTS = PDEPTH / ROWS;
   static_assert(SLOTS * ROWS == PDEPTH && RUN % ROWS == 0, "ring shape");
   extern __shared__ __align__(128) unsigned char smem64[];
@@ -513,18 +534,16 @@ __global__ void __launch_bounds__(MAXT, MINB)
   const unsigned wmask = wthreads == 32 ? 0xffffffffu : ((1u << wthreads) - 1u);
   const int NN = N * N;
   const long long KC2 = (long long)NN * N / 2;  // float4 per table row
-  // shared memory: [nwarps][SLOTS] mbarriers; [nwarps] refill cursors; B rings
-  // [nwarps][PDEPTH rows][32 threads][2 float4]; the neighbour-pair planes (hi,
-  // then lo) [N][N] float4
-  uint64_t *bars = reinterpret_cast<uint64_t *>(smem64);
-  P64Cursor *curs =
-      reinterpret_cast<P64Cursor *>(smem64 + 16 * ((nwarps * SLOTS * 8 + 15) / 16));
-  float4 *rings = reinterpret_cast<float4 *>(reinterpret_cast<unsigned char *>(curs) +
-                                             sizeof(P64Cursor) * nwarps);
-  float4 *ehi = rings + (TMA ? (size_t)nwarps * PDEPTH * 32 * 2 : 0);
+  // float4 of a ring row: a warp's segment (a CTA of under one warp at N < 12)
+  const int RS = NC > 0 ? 64 : 2 * min(32, (int)blockDim.x);
+  // shared memory: B rings [nwarps][PDEPTH rows][RS float4]; the neighbour-pair
+  // planes (hi, then lo) [N][N] float4; [nwarps][SLOTS] mbarriers
+  float4 *rings = reinterpret_cast<float4 *>(smem64);
+  float4 *ehi = rings + (TMA ? nwarps * PDEPTH * RS : 0);
   float4 *elo = ehi + NN;
+  uint64_t *bars = reinterpret_cast<uint64_t *>(elo + NN);
   uint64_t *mybar = bars + warp * SLOTS;
-  float4 *myring = rings + (size_t)warp * PDEPTH * 32 * 2;
+  float4 *myring = rings + warp * PDEPTH * RS;
 
   const int r = tid % R4;
   const int j2l = tid / R4;
@@ -553,53 +572,43 @@ __global__ void __launch_bounds__(MAXT, MINB)
   const int hsw = (int)((kcol >> 4) & 1);  // halves stored swapped
   const long long wcol = ((long long)j1 * N + (blockIdx.y * J2T + (warp * 32) / R4)) * N +
                          ((warp * 32) % R4) * RUN;
-  const uint32_t seg_bytes = (uint32_t)(wthreads * RUN * sizeof(float2));
   const int nrows = (c1 - c0) * N;  // a multiple of 4
   // a zero limit: every wait has run out at once
   bool to = TMA && wait_ns == 0;
-  // lane 0's cursor (kept in shared memory, off the registers of the loop):
-  // the next row to issue as (list plane, i2, i3), its source, and the fills
-  // issued so far
-  if (TMA && lane == 0) {
-    P64Cursor c;
-    c.issued = 0;
-    c.src = nullptr;
-    c.pi = c.i2 = c.i3 = 0;
-    if (PDEPTH < nrows) {
-      const int t = c0 + PDEPTH / N;
-      c.pi = t / N;
-      c.i2 = t % N;
-      c.i3 = PDEPTH % N;
-      c.src = B2p + (((long long)plane_i1(c.pi) * N + c.i2) * N + c.i3) * KC2 + wcol / 2;
+  // Refills, the same in all lanes: the next table row to copy (its box ends
+  // within the l-line, as ROWS divides N), the rows up to the end of its l1
+  // plane, and the rows of the chunk still to copy.
+  const uint32_t box_bytes = (uint32_t)(ROWS * RS * sizeof(float4));
+  const uint32_t ring_a = s_addr(myring), bar_a = s_addr(mybar);
+  int rf_pi = c0 / N, rf_row = (plane_i1(rf_pi) * N + c0 % N) * N;
+  int rf_end = (N - c0 % N) * N, rf_left = nrows;
+  auto refill = [&](int slot, bool good) {
+    const bool on = good && rf_left > 0;
+    box_g2s(ring_a + slot * box_bytes, &tmB, (int)(2 * wcol), rf_row, box_bytes,
+            bar_a + slot * 8, on && lane == 0);
+    if (on) {
+      rf_left -= ROWS;
+      rf_row += ROWS;
+      if ((rf_end -= ROWS) == 0) {
+        rf_end = NN;
+        rf_row = plane_i1(++rf_pi) * NN;
+      }
     }
-    curs[warp] = c;
-  }
-
+  };
   if (TMA) {
     if (lane == 0) {
       for (int d = 0; d < SLOTS; ++d) mbar_init(&mybar[d], 1);
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncwarp(wmask);
-    if (lane == 0) {  // prologue: rows [0, PDEPTH)
-      for (int s = 0; s < SLOTS && s * ROWS < nrows; ++s) {
-        const int nr = min(ROWS, nrows - s * ROWS);
-        mbar_expect_tx(&mybar[s], seg_bytes * nr);
-        for (int rr = 0; rr < nr; ++rr) {
-          const int qq = s * ROWS + rr;
-          bulk_g2s(myring + (size_t)qq * 32 * 2, B2p + row_of(qq) * KC2 + wcol / 2, seg_bytes,
-                   &mybar[s]);
-        }
-        ++curs[warp].issued;
-      }
-    }
+    for (int sl = 0; sl < SLOTS; ++sl) refill(sl, true);  // rows [0, PDEPTH)
   }
 
   DF2 accR[2], accI[2];  // lanes (j3_0 + 2h, j3_0 + 2h + 1)
 #pragma unroll
   for (int h = 0; h < 2; ++h) accR[h].h = accR[h].l = accI[h].h = accI[h].l = 0ull;
   const u64 MONE = pk(-1.0f, -1.0f);
-  const float4 *lring = myring + (size_t)lane * 2 + hsw;  // this lane's first half, ring row 0
+  const float4 *lring = myring + lane * 2 + hsw;  // this lane's first half, ring row 0
 
   int cur_i1 = -1;
   int q = 0;  // chunk row of the current group's first step (a multiple of 4)
@@ -656,41 +665,18 @@ __global__ void __launch_bounds__(MAXT, MINB)
 #pragma unroll(NC == 24 ? 2 : 1)
     for (int g = 0; g < N; g += RUN, q += RUN) {
       const int an = am == 0 ? R4 - 1 : am - 1;
-      const float4 *ring_g = lring + (size_t)(q & 4) * 64;  // ring row q mod 8 = (q & 4) + t
+      const float4 *ring_g = lring + (q & 4) * RS;  // ring row q mod 8 = (q & 4) + t
 #pragma unroll
       for (int t = 0; t < RUN; ++t) {
         if (TMA) {
           const int slot = ((q & 4) + t) / ROWS;
           if (t % ROWS == 0) mbar_wait_nz(&mybar[slot], (uint32_t)((q >> 3) & 1), to, wait_ns);
-          bv0 = ring_g[t * 64];
-          bv1 = ring_g[t * 64 + 1 - 2 * hsw];
+          bv0 = ring_g[t * RS];
+          bv1 = ring_g[t * RS + 1 - 2 * hsw];
           if (t % ROWS == ROWS - 1) {
             // every lane has read the slot's rows; refill it with the next
             // ROWS rows unless a lane timed out
-            const bool bad = __any_sync(wmask, to);
-            const int first = q + t + 1 - ROWS + PDEPTH;
-            if (lane == 0 && !bad && first < nrows) {
-              const int nr = min(ROWS, nrows - first);
-              P64Cursor c = curs[warp];
-              asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-              mbar_expect_tx(&mybar[slot], seg_bytes * nr);
-              for (int rr = 0; rr < nr; ++rr) {
-                bulk_g2s(myring + ((size_t)(slot * ROWS + rr) * 32) * 2, c.src, seg_bytes,
-                         &mybar[slot]);
-                if (++c.i3 == N) {
-                  c.i3 = 0;
-                  if (++c.i2 == N) {
-                    c.i2 = 0;
-                    ++c.pi;
-                  }
-                  c.src = B2p + ((long long)plane_i1(c.pi) * N + c.i2) * N * KC2 + wcol / 2;
-                } else {
-                  c.src += KC2;
-                }
-              }
-              ++c.issued;
-              curs[warp] = c;
-            }
+            refill(slot, !__any_sync(wmask, to));
           }
         } else if (g + t + 1 < N) {
           const float4 *bn = brow + (long long)(g + t + 1) * KC2;
@@ -738,7 +724,7 @@ __global__ void __launch_bounds__(MAXT, MINB)
         // drain: fill f went into slot f % SLOTS, and a slot is refilled only
         // after its previous fill landed, so only each slot's last fill can
         // still be in flight
-        const int issued = curs[warp].issued;
+        const int issued = (nrows - rf_left) / ROWS;
         for (int sl = 0; sl < SLOTS && sl < issued; ++sl) {
           const int last = sl + ((issued - 1 - sl) / SLOTS) * SLOTS;
           bool t2 = false;
@@ -776,8 +762,9 @@ struct C64xShape {
 constexpr C64xShape kC64xShapes[] = {{256, 2}, {256, 1}, {128, 3}, {128, 4}, {192, 2}};
 constexpr int kC64xNShapes = (int)(sizeof(kC64xShapes) / sizeof(kC64xShapes[0]));
 // The output-pair kernel's shapes (same count): CTA size bound, CTAs per SM,
-// table rows per ring slot.  N = 32 (ms per launch): 1.27, 1.37, 1.62, 1.54
-// for the first four with 4, 2, 2, 2 rows; 1.45 with one row per slot.
+// table rows per ring slot.  ms per sum, whole waves | schedule model:
+//   N = 24  0.285 0.285 0.295 0.287 0.307 | 0.262 0.277 0.376 0.326 0.295
+//   N = 32  1.052 1.162 1.261 1.329 1.212 | 1.093 1.174 1.103 1.153 1.175
 struct C64pShape {
   int maxt, minb, rows;
 };
@@ -786,17 +773,20 @@ static_assert(sizeof(kC64pShapes) / sizeof(kC64pShapes[0]) == kC64xNShapes, "sha
 // the output-pair kernel runs the pair table when N is a multiple of 4
 static bool c64_op(const QParams &p, bool paired) { return paired && p.N % RUN == 0; }
 
-// N fixed at compile time for the output-pair kernel's tensor-copy form at
-// these sizes (0: runtime N)
+// N fixed at compile time for the output-pair kernel's tensor-copy form from
+// N = 20 up (0: runtime N): N = 20 109 -> 105 us, N = 28 629 -> 605 us per sum;
+// at N = 16 40.3 us either way.
 static int c64_nc(const QParams &p, bool op, bool tma) {
-  return (op && tma && (p.N == 24 || p.N == 32)) ? p.N : 0;
+  return (op && tma && p.N >= 20 && p.N <= 32) ? p.N : 0;
 }
 template <bool TMA, int S>
 static const void *c64x_fn_s(bool op, int nc) {
   constexpr int T = kC64pShapes[S].maxt, B = kC64pShapes[S].minb, R = kC64pShapes[S].rows;
   if (op) {
     if constexpr (TMA) {
+      if (nc == 20) return (const void *)calq64p_kernel<TMA, T, B, R, 20>;
       if (nc == 24) return (const void *)calq64p_kernel<TMA, T, B, R, 24>;
+      if (nc == 28) return (const void *)calq64p_kernel<TMA, T, B, R, 28>;
       if (nc == 32) return (const void *)calq64p_kernel<TMA, T, B, R, 32>;
     }
     return (const void *)calq64p_kernel<TMA, T, B, R, 0>;
@@ -817,8 +807,8 @@ static const void *c64x_fn(int shape, bool op, int nc) {
 static size_t c64x_smem(int N, int threads, bool tma, bool op, int rows) {
   const int nwarps = (threads + 31) / 32;
   if (op) {
-    size_t o = 16 * (size_t)((nwarps * (PDEPTH / rows) * 8 + 15) / 16) + sizeof(P64Cursor) * nwarps;
-    if (tma) o += 2 * sizeof(float4) * (size_t)nwarps * PDEPTH * 32;
+    size_t o = (size_t)nwarps * (PDEPTH / rows) * 8;
+    if (tma) o += 2 * sizeof(float4) * (size_t)nwarps * PDEPTH * std::min(32, threads);
     return o + 2 * sizeof(float4) * (size_t)N * N;
   }
   size_t o = 16 * (size_t)((nwarps * DEPTH * 8 + 15) / 16);
@@ -894,8 +884,8 @@ static C64xPlan c64x_plan_compute(const QParams &p, bool aligned, int shape_in, 
   // then the chunk) on the `wave` resident slots, each as soon as a slot
   // frees, and cost their own lines plus a quarter line; efficiency = useful
   // lines / (makespan * wave).  Neither predicts every table: measured at
-  // N = 24 the model's plan is 4% faster, at N = 32 3% slower (1.163 against
-  // 1.133 ms), so genB times both.
+  // N = 24 the model's plan is 8% faster, at N = 32 4% slower (1.093 against
+  // 1.052 ms), so genB times both.
   double best_eff = -1.0;
   int best_lc = NL;
   for (int ch = 1; ch <= NL; ++ch) {
@@ -973,26 +963,20 @@ int calq64x_shapes() { return 2 * kC64xNShapes; }
 template <bool TMA, int S>
 static void c64x_launch_s(dim3 grid, const C64xPlan &pl, const QParams &p, bool paired,
                           const float2 *d_B2, const float4 *d_fdf, double2 *d_partial,
-                          cudaStream_t st) {
+                          const CUtensorMap &tm, cudaStream_t st) {
   constexpr int T = kC64pShapes[S].maxt, B = kC64pShapes[S].minb, R = kC64pShapes[S].rows;
   const float4 *B2p = reinterpret_cast<const float4 *>(d_B2);
   if (c64_op(p, paired)) {
     const int nc = c64_nc(p, true, TMA);
-    bool done = false;
+    auto *fn = calq64p_kernel<TMA, T, B, R, 0>;
     if constexpr (TMA) {
-      if (nc == 24) {
-        calq64p_kernel<TMA, T, B, R, 24><<<grid, pl.threads, pl.smem, st>>>(
-            p, pl.J2T, pl.LC, B2p, d_fdf, d_partial, wait_limit_ns());
-        done = true;
-      } else if (nc == 32) {
-        calq64p_kernel<TMA, T, B, R, 32><<<grid, pl.threads, pl.smem, st>>>(
-            p, pl.J2T, pl.LC, B2p, d_fdf, d_partial, wait_limit_ns());
-        done = true;
-      }
+      if (nc == 20) fn = calq64p_kernel<TMA, T, B, R, 20>;
+      if (nc == 24) fn = calq64p_kernel<TMA, T, B, R, 24>;
+      if (nc == 28) fn = calq64p_kernel<TMA, T, B, R, 28>;
+      if (nc == 32) fn = calq64p_kernel<TMA, T, B, R, 32>;
     }
-    if (!done)
-      calq64p_kernel<TMA, T, B, R, 0><<<grid, pl.threads, pl.smem, st>>>(
-          p, pl.J2T, pl.LC, B2p, d_fdf, d_partial, wait_limit_ns());
+    fn<<<grid, pl.threads, pl.smem, st>>>(p, pl.J2T, pl.LC, B2p, d_fdf, d_partial,
+                                          wait_limit_ns(), tm);
   } else
     calq64x_kernel<TMA, kC64xShapes[S].maxt, kC64xShapes[S].minb>
         <<<grid, pl.threads, pl.smem, st>>>(p, pl.J2T, pl.LC, paired, d_B2, d_fdf, d_partial,
@@ -1001,13 +985,13 @@ static void c64x_launch_s(dim3 grid, const C64xPlan &pl, const QParams &p, bool 
 template <bool TMA>
 static void c64x_launch(int shape, dim3 grid, const C64xPlan &pl, const QParams &p, bool paired,
                         const float2 *d_B2, const float4 *d_fdf, double2 *d_partial,
-                        cudaStream_t st) {
+                        const CUtensorMap &tm, cudaStream_t st) {
   switch (shape) {
-    case 0: c64x_launch_s<TMA, 0>(grid, pl, p, paired, d_B2, d_fdf, d_partial, st); break;
-    case 1: c64x_launch_s<TMA, 1>(grid, pl, p, paired, d_B2, d_fdf, d_partial, st); break;
-    case 2: c64x_launch_s<TMA, 2>(grid, pl, p, paired, d_B2, d_fdf, d_partial, st); break;
-    case 3: c64x_launch_s<TMA, 3>(grid, pl, p, paired, d_B2, d_fdf, d_partial, st); break;
-    default: c64x_launch_s<TMA, 4>(grid, pl, p, paired, d_B2, d_fdf, d_partial, st); break;
+    case 0: c64x_launch_s<TMA, 0>(grid, pl, p, paired, d_B2, d_fdf, d_partial, tm, st); break;
+    case 1: c64x_launch_s<TMA, 1>(grid, pl, p, paired, d_B2, d_fdf, d_partial, tm, st); break;
+    case 2: c64x_launch_s<TMA, 2>(grid, pl, p, paired, d_B2, d_fdf, d_partial, tm, st); break;
+    case 3: c64x_launch_s<TMA, 3>(grid, pl, p, paired, d_B2, d_fdf, d_partial, tm, st); break;
+    default: c64x_launch_s<TMA, 4>(grid, pl, p, paired, d_B2, d_fdf, d_partial, tm, st); break;
   }
 }
 
@@ -1029,10 +1013,19 @@ edb_status launch_calq64x(const QParams &p, const float2 *d_B2, const double2 *d
     return fail(EDB_EINVAL, "calq64x: the output-pair table must be 16-byte aligned");
   const C64xPlan pl = c64x_plan(p, aligned, shape, paired);
   dim3 grid((unsigned)p.P, (unsigned)pl.tiles, (unsigned)pl.nch);
+  CUtensorMap tm = {};
+  if (pl.tma && c64_op(p, paired)) {
+    const cuuint64_t dim[2] = {(cuuint64_t)(2 * p.NQ), (cuuint64_t)p.NQ};
+    const cuuint64_t str[1] = {(cuuint64_t)(8 * p.NQ)};
+    const cuuint32_t box[2] = {(cuuint32_t)(8 * std::min(32, pl.threads)),
+                               (cuuint32_t)kC64pShapes[shape % kC64xNShapes].rows};
+    if (!encode_map(&tm, 2, d_B2, dim, str, box))
+      return fail(EDB_ECUDA, "calq64x: cuTensorMapEncodeTiled");
+  }
   if (pl.tma)
-    c64x_launch<true>(shape % kC64xNShapes, grid, pl, p, paired, d_B2, d_fdf, d_partial, st);
+    c64x_launch<true>(shape % kC64xNShapes, grid, pl, p, paired, d_B2, d_fdf, d_partial, tm, st);
   else
-    c64x_launch<false>(shape % kC64xNShapes, grid, pl, p, paired, d_B2, d_fdf, d_partial, st);
+    c64x_launch<false>(shape % kC64xNShapes, grid, pl, p, paired, d_B2, d_fdf, d_partial, tm, st);
   EDB_LAUNCHED();
   return launch_calq64_reduce(p, pl.nch, d_partial, d_Q, st);
 }

@@ -1,0 +1,46 @@
+"""The table copies of the double-float sum at N % 4 == 0.
+
+Sizes: CTAs of under one warp (N = 4, 8), with a last warp that is partly empty
+(N = 12, 20, 24, 28) and of full warps (N = 16); every launch shape, so every
+number of rows a copy, and both rules for the l-line chunks.
+
+Tolerance: the drop-in path's bound, relative L2 <= 1e-12.
+"""
+import numpy as np
+import pytest
+
+from oracle.oracle import INDEX_ALIASED
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def edb():
+    import entropydecreaseboltzmann_gb300 as e
+
+    return e
+
+
+@pytest.mark.parametrize("N", [4, 8, 12, 16, 20, 24, 28])
+def test_every_launch_shape_against_the_direct_sum(edb, oracle, N):
+    L = 6.0
+    rng = np.random.default_rng(N)
+    fin = rng.standard_normal(N ** 3) + 1j * rng.standard_normal(N ** 3)
+    modes = rng.choice(N ** 3, min(N ** 3, 96), replace=False)
+    modes[:2] = 0, N ** 3 - 1
+    want = oracle.direct_modes(N, fin, modes, gamma=0.0, R=L, filter=False)
+    q = edb.QCalculator(N, 0, L=L, filter=False, index_mode=INDEX_ALIASED)
+    q.genB()
+    for shape in range(edb.lib.edb_qcalc_fp64_shapes()):
+        q.fp64_shape(shape)
+        got = q.calQ(None, fin)[modes]
+        assert np.linalg.norm(got - want) <= 1e-12 * np.linalg.norm(want), shape
+    # a wait that runs out is reported, and the next call is whole again
+    edb.set_wait_limit_ns(0)
+    try:
+        with pytest.raises(edb.EdbError) as e:
+            q.calQ(None, fin)
+        assert e.value.status == 4
+    finally:
+        edb.set_wait_limit_ns(-1)
+    assert np.array_equal(q.calQ(None, fin)[modes], got)
