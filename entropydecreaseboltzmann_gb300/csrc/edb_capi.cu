@@ -318,7 +318,7 @@ extern "C" edb_status edb_qcalc_genB(edb_qcalc *q) {
   double *T = nullptr, *sigma = nullptr, *Bmm = nullptr;
   edb_status s = EDB_OK;
   if (!q->B64) EDB_TRY(dalloc(&q->B64, (size_t)NQ * NQ));
-  if (!q->B2) EDB_TRY(dalloc(&q->B2, (size_t)NQ * NQ));
+  if (!q->B2) EDB_TRY(dalloc(&q->B2, (size_t)calq64x_table(q->p.N, qcalc_b2_paired(q))));
   if (q->d.index_mode == EDB_INDEX_ALIASED && !q->B32)
     EDB_TRY(dalloc(&q->B32, (size_t)c32_table_floats(N) + 64));  // +64: masked tail reads
   EDB_TRY(qcalc_alloc_work(q));
@@ -449,7 +449,7 @@ long long qcalc_table_bytes(const edb_qcalc *q) {
   long long b = 0;
   const long long e = q->p.NQ * q->p.NQ;
   if (q->B64) b += e * 8;
-  if (q->B2) b += e * 8;
+  if (q->B2) b += calq64x_table(q->p.N, qcalc_b2_paired(q)) * 8;
   if (q->B32) b += c32_table_floats(q->p.N) * 4 + 256;
   if (q->tc) b += (long long)(q->amax + 1) * calq64f_row_len(q->amax) * 8 + q->p.NQ * 16;
   return b;
@@ -462,7 +462,7 @@ extern "C" edb_status edb_qcalc_set_B(edb_qcalc *q, const double *host_B) {
   if (!q->B64) EDB_TRY(dalloc(&q->B64, (size_t)NQ * NQ));
   EDB_TRY(qcalc_alloc_work(q));
   EDB_CUDA(cudaMemcpy(q->B64, host_B, sizeof(double) * NQ * NQ, cudaMemcpyHostToDevice));
-  if (!q->B2) EDB_TRY(dalloc(&q->B2, (size_t)NQ * NQ));
+  if (!q->B2) EDB_TRY(dalloc(&q->B2, (size_t)calq64x_table(q->p.N, qcalc_b2_paired(q))));
   EDB_TRY(qcalc_split_B2(q));
   EDB_CUDA(cudaStreamSynchronize(q->st));
   dfree(q->B32);  // the FP32 copy no longer matches

@@ -67,6 +67,15 @@ __device__ __forceinline__ void df_axpy(DF2 &acc, u64 sh2, u64 nsh2, u64 nsl2, u
   acc.l = add2(acc.l, add2(e, pl));
 }
 
+// acc with its low part brought back under half a unit of the high one (Dekker's
+// sum; where the high part has cancelled to below the low one it is off by a
+// rounding of the low one, as any addition to that is).
+__device__ __forceinline__ void df_renorm(DF2 &acc) {
+  const u64 s = add2(acc.h, acc.l);
+  acc.l = sub2(acc.l, sub2(s, acc.h));
+  acc.h = s;
+}
+
 // ---- scalar {hi, lo}
 // a + b = s + e exactly (Knuth)
 __device__ __forceinline__ float2 two_sum(float a, float b) {

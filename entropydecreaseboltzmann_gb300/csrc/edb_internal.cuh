@@ -132,6 +132,8 @@ int calq64x_nchunk(const QParams &p, int *J2T_out);
 // false: the driver has no encoder or refused the map.
 bool encode_map(CUtensorMap *m, int rank, const void *base, const cuuint64_t *dim,
                 const cuuint64_t *stride, const cuuint32_t *box);
+// Entries (float2) of B2; the pair table's rows are padded to whole fours of k3.
+long long calq64x_table(int N, bool paired);
 edb_status launch_split_f(long long n, const double2 *f, float4 *out, cudaStream_t st);
 edb_status launch_split_B(long long n, const double *B, float2 *B2, cudaStream_t st);
 // ALIASED tables: B2 = split of the symmetric pair table (B[l][k] + B[k-l][k]

@@ -27,9 +27,9 @@
 // Pairs: with the aliased index shifts (ALIASED mode, or odd N) B2 is the
 // split symmetric pair table (b2_pair_split_kernel) and each output plane
 // visits only the l1 planes with l1 <= (k1 - l1) mod N, about half the B
-// stream; otherwise every l-line is visited with B split as it is.  When N is
-// a multiple of 4 the pair table is read by calq64p_kernel instead (the same
-// sum with neighbouring outputs in the packed lanes; see there).
+// stream; calq64p_kernel reads it (the same sum with neighbouring outputs in the
+// packed lanes; see there).  Otherwise calq64x_kernel visits every l-line with B
+// split as it is.
 //
 // Tiling: CTA = (output plane j1, a tile of j2, all j3) x (a chunk of its
 // l-lines (i1, i2)).  Thread = (j2, run of 4 consecutive j3).  For each i1 the f-hat
@@ -40,11 +40,12 @@
 // FP64 partial sums per chunk; calq64_reduce_kernel adds the chunks in order.
 //
 // B stream: when every warp's row segment is a contiguous, 16-byte aligned run
-// (P % 4 == 0 and whole j2 tiles), each warp streams its own 1 KB segment of
-// the next D rows into a private shared-memory ring with TMA copies (1-D bulk
-// copies here, boxes of rows in calq64p_kernel; lane 0 issues; one mbarrier per
-// slot; waits bounded by %globaltimer, a timeout sets the device status word).  Otherwise threads load their 32
-// bytes per row with __ldg, one row ahead.
+// (calq64p_kernel always; here P % 4 == 0 and whole j2 tiles), each warp streams
+// its own 1 KB segment of the next D rows into a private shared-memory ring with
+// TMA copies (boxes of rows there, 1-D bulk copies here; lane 0 issues; one
+// mbarrier per slot; waits bounded by %globaltimer, a timeout sets the device
+// status word).  Otherwise threads load their 32 bytes per row with __ldg, one
+// row ahead.
 #include <cuda.h>
 
 #include <algorithm>
@@ -196,32 +197,32 @@ __global__ void b2_split_kernel(long long n, const double *__restrict__ B, float
 // m_d = (k_d - l_d + n) mod N, summed in FP64 and then split, or B[l][k]
 // alone when l and m share the first index (both terms lie on one visited
 // plane).  The terms l and m of a Q-hat sum carry the same product f_l f_m.
+// Layout (calq64p_kernel): k3 padded with zeros to N4, the next multiple of
+// four; each aligned group G of four entries of a row as the halves
+// {h0, h1, l0, l1}, {h2, h3, l2, l3}, in swapped order when bit 2 of G is set
+// (the reader's 128-bit loads then spread over all bank groups).
 __global__ void b2_pair_split_kernel(int N, const double *__restrict__ B, float2 *__restrict__ B2) {
-  const long long NQ = (long long)N * N * N;
+  const int N4 = (N + RUN - 1) / RUN * RUN;
+  const long long NQ = (long long)N * N * N, KP = (long long)N * N * N4;
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= NQ * NQ) return;
-  const long long l = i / NQ, k = i - l * NQ;
+  if (i >= NQ * KP) return;
+  const long long l = i / KP, kp = i - l * KP;
   const int n = (N - 1) / 2;
   const int l1 = (int)(l / (N * N)), l2 = (int)((l / N) % N), l3 = (int)(l % N);
-  const int k1 = (int)(k / (N * N)), k2 = (int)((k / N) % N), k3 = (int)(k % N);
-  const int m1 = (k1 - l1 + n + N) % N, m2 = (k2 - l2 + n + N) % N, m3 = (k3 - l3 + n + N) % N;
-  double v = B[i];
-  if (m1 != l1) v += B[(((long long)m1 * N + m2) * N + m3) * NQ + k];
-  const float h = (float)v;
-  const float lo = (float)(v - (double)h);
-  if (N % RUN == 0) {
-    // output-pair layout (calq64p_kernel): each aligned group G of four
-    // entries as the halves {h0, h1, l0, l1}, {h2, h3, l2, l3}, in swapped
-    // order when bit 2 of G is set (the reader's 128-bit loads then spread
-    // over all bank groups)
-    float *o = reinterpret_cast<float *>(B2);
-    const long long half = ((i >> 1) & 1) ^ ((i >> 4) & 1);
-    const long long hp = 2 * (i & ~3ll) + half * 4 + (i & 1);
-    o[hp] = h;
-    o[hp + 2] = lo;
-  } else {
-    B2[i] = make_float2(h, lo);
+  const int k1 = (int)(kp / (N * N4)), k2 = (int)((kp / N4) % N), k3 = (int)(kp % N4);
+  double v = 0.0;
+  if (k3 < N) {
+    const int m1 = (k1 - l1 + n + N) % N, m2 = (k2 - l2 + n + N) % N, m3 = (k3 - l3 + n + N) % N;
+    const long long k = ((long long)k1 * N + k2) * N + k3;
+    v = B[l * NQ + k];
+    if (m1 != l1) v += B[(((long long)m1 * N + m2) * N + m3) * NQ + k];
   }
+  const float h = (float)v;
+  float *o = reinterpret_cast<float *>(B2 + l * KP);
+  const long long half = ((kp >> 1) & 1) ^ ((kp >> 4) & 1);
+  const long long hp = 2 * (kp & ~3ll) + half * 4 + (kp & 1);
+  o[hp] = h;
+  o[hp + 2] = (float)(v - (double)h);
 }
 
 // TMA: per-warp bulk-copy ring for B (requires contiguous, aligned warp
@@ -232,7 +233,7 @@ __global__ void b2_pair_split_kernel(int N, const double *__restrict__ B, float2
 // table by timing every shape (edb_qcalc_genB runs the comparison once).
 template <bool TMA, int MAXT, int MINB>
 __global__ void __launch_bounds__(MAXT, MINB)
-    calq64x_kernel(QParams p, int J2T, int LC, int paired, const float2 *__restrict__ B2,
+    calq64x_kernel(QParams p, int J2T, int LC, const float2 *__restrict__ B2,
                    const float4 *__restrict__ fdf, double2 *__restrict__ partial,
                    unsigned long long wait_ns) {
   extern __shared__ __align__(128) unsigned char smem64[];
@@ -259,25 +260,8 @@ __global__ void __launch_bounds__(MAXT, MINB)
   const int j2c = ok ? j2 : 0;
   const int j3_0 = r * RUN;
   const int chunk = blockIdx.z;
-  // l1 planes this output plane visits.  Paired table (ALIASED): the terms l
-  // and m = k - l share the product f_l f_m and B2 holds B[l][k] + B[m][k], so
-  // only the planes with a1 <= (k1 - a1) mod N are visited (a1, k1 in FFTW
-  // order): [0, k1/2] and [k1+1, (k1+N)/2].  Otherwise every i1 in order.
-  const int k1f = (j1 - p.n + N) % N;
-  const int plo = k1f / 2;
-  const int nlist = paired ? plo + 1 + max(0, (k1f + N) / 2 - k1f) : N;
-  auto plane_i1 = [&](int pi) {
-    if (!paired) return pi;
-    const int a = pi <= plo ? pi : k1f + 1 + (pi - plo - 1);
-    return (a + p.n) % N;  // a = (i1 - n) mod N
-  };
-  const int NL = nlist * N;  // l-lines (i1, i2) of those planes
+  const int NL = N * N;  // l-lines (i1, i2)
   const int c0 = min(NL, chunk * LC), c1 = min(NL, c0 + LC);
-  // B2 row of the chunk's qq-th row (line c0 + qq / N, i3 = qq mod N)
-  auto row_of = [&](int qq) -> long long {
-    const int t = c0 + qq / N;
-    return ((long long)plane_i1(t / N) * N + t % N) * N + qq % N;
-  };
   const long long kcol = ((long long)j1 * P + j2c) * P + j3_0;
   // columns past P (ragged last run) read a clamped, in-row column and are
   // masked out of the output
@@ -293,19 +277,8 @@ __global__ void __launch_bounds__(MAXT, MINB)
   const int nrows = (c1 - c0) * N;  // rows this CTA streams
   bool to = false;
   int issued = 0;  // lane 0: rows its warp has issued into the ring
-  // refill cursor (lane 0): row q + DEPTH of the chunk as (list plane, i2, i3),
-  // advanced by one row per refill so the per-row path has no division
-  int rf_pi = 0, rf_i2 = 0, rf_i3 = 0;
-  long long rf_base = 0;
-  const float2 *rf_src = nullptr;  // source of row q + DEPTH: B2 + (rf_base + rf_i3) KC + wcol
-  if (TMA && lane == 0 && DEPTH < nrows) {
-    const int t = c0 + DEPTH / N;
-    rf_pi = t / N;
-    rf_i2 = t % N;
-    rf_i3 = DEPTH % N;
-    rf_base = ((long long)plane_i1(rf_pi) * N + rf_i2) * N;
-    rf_src = B2 + (rf_base + rf_i3) * p.KC + wcol;
-  }
+  // the chunk's rows follow one another in the table
+  const float2 *rf_src = B2 + (long long)c0 * N * p.KC + wcol;  // next row to copy
 
   if (TMA) {
     if (lane == 0) {
@@ -315,9 +288,9 @@ __global__ void __launch_bounds__(MAXT, MINB)
     __syncwarp(wmask);
     if (lane == 0) {  // prologue: the first DEPTH rows
       for (int q = 0; q < DEPTH && q < nrows; ++q) {
-        const long long lflat = row_of(q);
         mbar_expect_tx(&mybar[q], seg_bytes);
-        bulk_g2s(myring + (size_t)q * 32 * RUN, B2 + lflat * p.KC + wcol, seg_bytes, &mybar[q]);
+        bulk_g2s(myring + (size_t)q * 32 * RUN, rf_src, seg_bytes, &mybar[q]);
+        rf_src += p.KC;
         ++issued;
       }
     }
@@ -338,7 +311,7 @@ __global__ void __launch_bounds__(MAXT, MINB)
     // line indices: i1, i2 (centred l); a1, a2 = (i + sL) mod N (f_l, FFTW
     // order); m2 = (j2 - i2 + sM) mod N.  Computed per line: counters kept
     // across the loop cost registers and measured slower here.
-    const int i1 = plane_i1(line / N), i2 = line % N;
+    const int i1 = line / N, i2 = line % N;
     const int a1 = (i1 + p.sL) % N, a2 = (i2 + p.sL) % N;
     const int m2 = ((j2c - i2 + p.sM) % N + N) % N;
     if (i1 != cur_i1) {  // stage the m1-plane
@@ -394,19 +367,7 @@ __global__ void __launch_bounds__(MAXT, MINB)
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             mbar_expect_tx(&mybar[slot], seg_bytes);
             bulk_g2s(myring + (size_t)slot * 32 * RUN, rf_src, seg_bytes, &mybar[slot]);
-            // the next row is one row of the table further (KC entries) within
-            // a line; a new line restarts from its own row block
-            if (++rf_i3 == N) {
-              rf_i3 = 0;
-              if (++rf_i2 == N) {
-                rf_i2 = 0;
-                ++rf_pi;
-              }
-              rf_base = ((long long)plane_i1(rf_pi) * N + rf_i2) * N;
-              rf_src = B2 + rf_base * p.KC + wcol;
-            } else {
-              rf_src += p.KC;
-            }
+            rf_src += p.KC;
             ++issued;
           }
         } else if (i3 + 1 < N) {
@@ -478,7 +439,7 @@ __global__ void __launch_bounds__(MAXT, MINB)
   }
 }
 
-// Output-pair form of calq64x_kernel (pair table, N % 4 == 0).  The f32x2
+// Output-pair form of calq64x_kernel, for the pair table.  The f32x2
 // lanes carry two neighbouring outputs (j3, j3 + 1) instead of the (re, im)
 // parts of one, so the table's values enter the packed instructions as they
 // are stored: each thread's four entries of a row are laid out as
@@ -495,7 +456,7 @@ __global__ void __launch_bounds__(MAXT, MINB)
 // at step i3 the pair (0, 1) reads E[x], the pair (2, 3) E[x + 2], x =
 // (j3_0 - i3 + sM) mod N, so one new entry per step and a ring of four.  The
 // hi and lo halves sit in two planes, each row stored transposed, E[x] at
-// (x mod 4) N/4 + x/4: the lanes of a row read x four apart, which then fall
+// (x mod 4) R4 + x/4, R4 runs of four to a row: the lanes of a row read x four apart, which then fall
 // in distinct 16-byte bank groups (at N = 32 every 128-bit load is
 // conflict-free; untransposed, eight lanes shared one group).
 // B stream: ROWS table rows per ring slot (one wait, one vote and one tensor
@@ -506,7 +467,23 @@ __global__ void __launch_bounds__(MAXT, MINB)
 // 51 -> 40 us, 20 125 -> 105, 24 286 -> 262, 28 704 -> 605, 32 1125 -> 1053),
 // against one copy of all ROWS rows, issued by predication, whose row number
 // every lane carries.
+// N not a multiple of four (RAG): the last run of a row has idle outputs, its
+// table entries zeros, so every row is whole fours, aligned, and its copies are
+// the same; a line takes its rows up to a multiple of four from the ring.  Read
+// by calq64x_kernel with plain loads one row ahead, the same pair table took:
+// N = 9 26.9 -> 22.7 us, 17 84 -> 70, 18 105 -> 85, 23 312 -> 260, 25 503 -> 417,
+// 27 757 -> 563, 31 1386 -> 1156.  That form kept the products with f_l.re and
+// f_l.im apart; one accumulator for both makes the low parts twice as long a
+// sum, so they are folded back every other step (3% of the time).  Relative
+// error against the FP64 kernel on near-equilibrium data, that form -> folded
+// (unfolded): N = 9 1.7e-14 -> 2.2e-14 (3.0e-14), 17 5.0e-14 -> 2.6e-14 (8.6e-14),
+// 23 9.1e-14 -> 3.6e-14 (1.6e-13), 30 6.7e-13 -> 6.8e-14 (6.5e-13).
 constexpr int PDEPTH = 8;
+// Threads whose entries one ring row holds: a warp's, or all of a CTA of under
+// one warp (N < 12), in fours so that a slot starts on a 128-byte boundary.
+__host__ __device__ constexpr int p64_box_threads(int threads) {
+  return threads >= 32 ? 32 : (threads + 3) / 4 * 4;
+}
 
 // fdr: f-hat split as for calq64x_kernel and rotated along the last axis by
 // the f_l shift, fdr[a1][a2][i] = f[a1][a2][(i + sL) mod N], with one float4 of
@@ -517,31 +494,30 @@ constexpr int PDEPTH = 8;
 // tmB: the table as N^3 rows of 2 N^3 floats, box ROWS rows of a full warp's
 // segment (the last warp, where it is short, copies a full box too: the columns
 // past its own are other threads' and are not read).
-template <bool TMA, int MAXT, int MINB, int ROWS, int NC>
+template <int MAXT, int MINB, int ROWS, int NC, bool RAG>
 __global__ void __launch_bounds__(MAXT, MINB)
-    calq64p_kernel(QParams p, int J2T, int LC, const float4 *__restrict__ B2p,
-                   const float4 *__restrict__ fdr, double2 *__restrict__ partial,
+    calq64p_kernel(QParams p, int J2T, int LC, const float4 *__restrict__ fdr, double2 *__restrict__ partial,
                    unsigned long long wait_ns, const __grid_constant__ CUtensorMap tmB) {
   constexpr int SLOTS = PDEPTH / ROWS;
   static_assert(SLOTS * ROWS == PDEPTH && RUN % ROWS == 0, "ring shape");
   extern __shared__ __align__(128) unsigned char smem64[];
   const int N = NC > 0 ? NC : p.N;  // == P
   const int n = (N - 1) / 2;
-  const int R4 = N / RUN;
+  const int R4 = RAG ? (N + RUN - 1) / RUN : N / RUN;
+  const int N4 = RAG ? R4 * RUN : N;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nwarps = (blockDim.x + 31) >> 5;
   const int wthreads = min(32, (int)blockDim.x - warp * 32);
   const unsigned wmask = wthreads == 32 ? 0xffffffffu : ((1u << wthreads) - 1u);
   const int NN = N * N;
-  const long long KC2 = (long long)NN * N / 2;  // float4 per table row
-  // float4 of a ring row: a warp's segment (a CTA of under one warp at N < 12)
-  const int RS = NC > 0 ? 64 : 2 * min(32, (int)blockDim.x);
+  // float4 of a ring row: a warp's segment (p64_box_threads threads)
+  const int RS = NC > 0 ? 64 : 2 * p64_box_threads(blockDim.x);
   // shared memory: B rings [nwarps][PDEPTH rows][RS float4]; the neighbour-pair
-  // planes (hi, then lo) [N][N] float4; [nwarps][SLOTS] mbarriers
+  // planes (hi, then lo) [N][N4] float4; [nwarps][SLOTS] mbarriers
   float4 *rings = reinterpret_cast<float4 *>(smem64);
-  float4 *ehi = rings + (TMA ? nwarps * PDEPTH * RS : 0);
-  float4 *elo = ehi + NN;
-  uint64_t *bars = reinterpret_cast<uint64_t *>(elo + NN);
+  float4 *ehi = rings + nwarps * PDEPTH * RS;
+  float4 *elo = ehi + N * N4;
+  uint64_t *bars = reinterpret_cast<uint64_t *>(elo + N * N4);
   uint64_t *mybar = bars + warp * SLOTS;
   float4 *myring = rings + warp * PDEPTH * RS;
 
@@ -563,46 +539,51 @@ __global__ void __launch_bounds__(MAXT, MINB)
   };
   const int NL = nlist * N;
   const int c0 = min(NL, chunk * LC), c1 = min(NL, c0 + LC);
-  auto row_of = [&](int qq) -> long long {
-    const int t = c0 + qq / N;
-    return ((long long)plane_i1(t / N) * N + t % N) * N + qq % N;
-  };
-  // entry index of the thread's run within a row (a multiple of 4: float4 kcol / 2)
-  const long long kcol = ((long long)j1 * N + j2c) * N + j3_0;
+  // entry index of the thread's run within a row (a multiple of 4)
+  const long long kcol = ((long long)j1 * N + j2c) * N4 + j3_0;
   const int hsw = (int)((kcol >> 4) & 1);  // halves stored swapped
-  const long long wcol = ((long long)j1 * N + (blockIdx.y * J2T + (warp * 32) / R4)) * N +
-                         ((warp * 32) % R4) * RUN;
-  const int nrows = (c1 - c0) * N;  // a multiple of 4
+  const long long wcol = ((long long)j1 * N + (blockIdx.y * J2T + (warp * 32) / R4)) * N4 +
+                   ((warp * 32) % R4) * RUN;
+  // ring rows of the chunk: RAG copies a line's rows up to a multiple of four,
+  // the rows past its N being the next line's (or zeros past the table), unused
+  const int nrows = (c1 - c0) * N4;
   // a zero limit: every wait has run out at once
-  bool to = TMA && wait_ns == 0;
-  // Refills, the same in all lanes: the next table row to copy (its box ends
-  // within the l-line, as ROWS divides N), the rows up to the end of its l1
-  // plane, and the rows of the chunk still to copy.
+  bool to = wait_ns == 0;
+  // Refills, the same in all lanes: the next table row to copy, the ring rows up
+  // to the end of its l1 plane (RAG: of its line, and that line's i2), and the
+  // ring rows of the chunk still to copy.
   const uint32_t box_bytes = (uint32_t)(ROWS * RS * sizeof(float4));
   const uint32_t ring_a = s_addr(myring), bar_a = s_addr(mybar);
-  int rf_pi = c0 / N, rf_row = (plane_i1(rf_pi) * N + c0 % N) * N;
-  int rf_end = (N - c0 % N) * N, rf_left = nrows;
+  int rf_pi = c0 / N, rf_i2 = c0 % N, rf_row = (plane_i1(rf_pi) * N + rf_i2) * N;
+  int rf_end = RAG ? N4 : (N - rf_i2) * N, rf_left = nrows;
   auto refill = [&](int slot, bool good) {
     const bool on = good && rf_left > 0;
-    box_g2s(ring_a + slot * box_bytes, &tmB, (int)(2 * wcol), rf_row, box_bytes,
-            bar_a + slot * 8, on && lane == 0);
+    box_g2s(ring_a + slot * box_bytes, &tmB, (int)(2 * wcol), rf_row, box_bytes, bar_a + slot * 8,
+            on && lane == 0);
     if (on) {
       rf_left -= ROWS;
       rf_row += ROWS;
       if ((rf_end -= ROWS) == 0) {
-        rf_end = NN;
-        rf_row = plane_i1(++rf_pi) * NN;
+        if constexpr (RAG) {
+          rf_end = N4;
+          rf_row -= N4 - N;
+          if (++rf_i2 == N) {
+            rf_i2 = 0;
+            rf_row = plane_i1(++rf_pi) * NN;
+          }
+        } else {
+          rf_end = NN;
+          rf_row = plane_i1(++rf_pi) * NN;
+        }
       }
     }
   };
-  if (TMA) {
-    if (lane == 0) {
-      for (int d = 0; d < SLOTS; ++d) mbar_init(&mybar[d], 1);
-      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncwarp(wmask);
-    for (int sl = 0; sl < SLOTS; ++sl) refill(sl, true);  // rows [0, PDEPTH)
+  if (lane == 0) {
+    for (int d = 0; d < SLOTS; ++d) mbar_init(&mybar[d], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  __syncwarp(wmask);
+  for (int sl = 0; sl < SLOTS; ++sl) refill(sl, true);  // rows [0, PDEPTH)
 
   DF2 accR[2], accI[2];  // lanes (j3_0 + 2h, j3_0 + 2h + 1)
 #pragma unroll
@@ -610,8 +591,10 @@ __global__ void __launch_bounds__(MAXT, MINB)
   const u64 MONE = pk(-1.0f, -1.0f);
   const float4 *lring = myring + lane * 2 + hsw;  // this lane's first half, ring row 0
 
+  // RAG: (4r + 1) mod N and (4r + 2) mod N (N may be under 3)
+  const int x1 = RAG ? (j3_0 + 1) % N : 0, x2 = RAG ? (j3_0 + 2) % N : 0;
   int cur_i1 = -1;
-  int q = 0;  // chunk row of the current group's first step (a multiple of 4)
+  int q = 0;  // ring row of the current group's first step (a multiple of 4)
   for (int line = c0; line < c1; ++line) {
     const int i1 = plane_i1(line / N), i2 = line % N;
     // f_l row (a1, a2) = (i + sL) mod N with sL = N - n; m = k - l for k1 = j1, k2 = j2
@@ -629,7 +612,7 @@ __global__ void __launch_bounds__(MAXT, MINB)
         if (cr >= N) cr -= N;
         const int cr1 = cr + 1 == N ? 0 : cr + 1;
         const float4 v0 = src[row * N + cr], v1 = src[row * N + cr1];
-        const int d = row * N + (c & 3) * R4 + (c >> 2);
+        const int d = row * N4 + (c & 3) * R4 + (c >> 2);
         ehi[d] = make_float4(v0.x, v1.x, v0.y, v1.y);
         elo[d] = make_float4(v0.z, v1.z, v0.w, v1.w);
       }
@@ -637,10 +620,9 @@ __global__ void __launch_bounds__(MAXT, MINB)
     }
     // E[x] of the row at (x mod 4) R4 + x / 4.  Step i3 = g + t reads
     // x = (4r - i3) mod N: x / 4 = a (the group's a) at t = 0, and for t >= 1
-    // x mod 4 = 4 - t with x / 4 = (a - 1) mod R4.
-    const float4 *erh = ehi + m2 * N, *erl = elo + m2 * N;
+    // x mod 4 = 4 - t with x / 4 = (a - 1) mod R4.  RAG: x itself steps down.
+    const float4 *erh = ehi + m2 * N4, *erl = elo + m2 * N4;
     const float4 *flp = fdr + ((long long)a1 * N + a2) * N;
-    const long long lrow0 = ((long long)i1 * N + i2) * N;
     u64 eh[4][2], el[4][2];  // ring[s]: E entry of step i3 with i3 mod 4 = s
     auto load_e = [&](int px, int s) {
       const float4 u = erh[px], w = erl[px];
@@ -649,15 +631,16 @@ __global__ void __launch_bounds__(MAXT, MINB)
       el[s][0] = pk(w.x, w.y);
       el[s][1] = pk(w.z, w.w);
     };
-    load_e(r, 0);           // x = 4r
-    load_e(R4 + r, 3);      // x = 4r + 1: E[x + 1] of step 0 = the entry of step -1
-    load_e(2 * R4 + r, 2);  // x = 4r + 2: E[x + 2] of step 0 = the entry of step -2
-    const float4 *brow = B2p + lrow0 * KC2 + kcol / 2;
-    float4 bv0, bv1, bn0, bn1;
-    if (!TMA) {
-      bv0 = __ldg(brow + hsw);
-      bv1 = __ldg(brow + 1 - hsw);
+    auto px_of = [&](int x) { return (x & 3) * R4 + (x >> 2); };
+    load_e(r, 0);  // x = 4r
+    if constexpr (RAG) {
+      load_e(px_of(x1), 3);
+      load_e(px_of(x2), 2);
+    } else {
+      load_e(R4 + r, 3);      // x = 4r + 1: E[x + 1] of step 0 = the entry of step -1
+      load_e(2 * R4 + r, 2);  // x = 4r + 2: E[x + 2] of step 0 = the entry of step -2
     }
+    int x = j3_0;
     float4 fl_next = __ldg(flp);
     int am = r;
     // at N = 24 two groups per iteration (0.304 -> 0.298 ms per launch); at
@@ -668,22 +651,20 @@ __global__ void __launch_bounds__(MAXT, MINB)
       const float4 *ring_g = lring + (q & 4) * RS;  // ring row q mod 8 = (q & 4) + t
 #pragma unroll
       for (int t = 0; t < RUN; ++t) {
-        if (TMA) {
-          const int slot = ((q & 4) + t) / ROWS;
-          if (t % ROWS == 0) mbar_wait_nz(&mybar[slot], (uint32_t)((q >> 3) & 1), to, wait_ns);
-          bv0 = ring_g[t * RS];
-          bv1 = ring_g[t * RS + 1 - 2 * hsw];
-          if (t % ROWS == ROWS - 1) {
-            // every lane has read the slot's rows; refill it with the next
-            // ROWS rows unless a lane timed out
-            refill(slot, !__any_sync(wmask, to));
+        const int slot = ((q & 4) + t) / ROWS;
+        if (t % ROWS == 0) mbar_wait_nz(&mybar[slot], (uint32_t)((q >> 3) & 1), to, wait_ns);
+        const float4 bv0 = ring_g[t * RS];
+        const float4 bv1 = ring_g[t * RS + 1 - 2 * hsw];
+        // every lane has read the slot's rows; refill it with the next ROWS
+        // rows unless a lane timed out
+        if (t % ROWS == ROWS - 1) refill(slot, !__any_sync(wmask, to));
+        if (RAG && g + t >= N) continue;
+        if constexpr (RAG) {
+          if (g + t > 0) {
+            x = x == 0 ? N - 1 : x - 1;
+            load_e(px_of(x), t);
           }
-        } else if (g + t + 1 < N) {
-          const float4 *bn = brow + (long long)(g + t + 1) * KC2;
-          bn0 = __ldg(bn + hsw);
-          bn1 = __ldg(bn + 1 - hsw);
-        }
-        if (t == 0) {
+        } else if (t == 0) {
           if (g > 0) load_e(am, 0);
         } else {
           load_e((4 - t) * R4 + an, t);
@@ -709,40 +690,45 @@ __global__ void __launch_bounds__(MAXT, MINB)
           df_axpy(accI[h], xr, nxr, nlr, nuim, ucim);  // + f_l.re u.im
           df_axpy(accI[h], xi, nxi, nli, nure, ucre);  // + f_l.im u.re
         }
-        if (!TMA) {
-          bv0 = bn0;
-          bv1 = bn1;
+        if (RAG && t % 2 == 1) {  // see above
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            df_renorm(accR[h]);
+            df_renorm(accI[h]);
+          }
         }
       }
       am = an;
     }
   }
-  if (TMA) {
-    if (__syncthreads_or(to)) {
-      if (lane == 0) {
-        atomicExch(&g_calq64x_status, 1);
-        // drain: fill f went into slot f % SLOTS, and a slot is refilled only
-        // after its previous fill landed, so only each slot's last fill can
-        // still be in flight
-        const int issued = (nrows - rf_left) / ROWS;
-        for (int sl = 0; sl < SLOTS && sl < issued; ++sl) {
-          const int last = sl + ((issued - 1 - sl) / SLOTS) * SLOTS;
-          bool t2 = false;
-          mbar_wait(&mybar[sl], (uint32_t)((last / SLOTS) & 1), t2, DRAIN_LIMIT_NS);
-        }
+  if (__syncthreads_or(to)) {
+    if (lane == 0) {
+      atomicExch(&g_calq64x_status, 1);
+      // drain: fill f went into slot f % SLOTS, and a slot is refilled only
+      // after its previous fill landed, so only each slot's last fill can
+      // still be in flight
+      const int issued = (nrows - rf_left) / ROWS;
+      for (int sl = 0; sl < SLOTS && sl < issued; ++sl) {
+        const int last = sl + ((issued - 1 - sl) / SLOTS) * SLOTS;
+        bool t2 = false;
+        mbar_wait(&mybar[sl], (uint32_t)((last / SLOTS) & 1), t2, DRAIN_LIMIT_NS);
       }
-      __syncwarp(wmask);
-      return;
     }
+    __syncwarp(wmask);
+    return;
   }
   if (!ok) return;
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     const float2 Rh = upk(accR[h].h), Rl = upk(accR[h].l);
     const float2 Ih = upk(accI[h].h), Il = upk(accI[h].l);
-    double2 *o = partial + (long long)chunk * NN * N + kcol + 2 * h;
-    o[0] = make_double2((double)Rh.x + (double)Rl.x, (double)Ih.x + (double)Il.x);
-    o[1] = make_double2((double)Rh.y + (double)Rl.y, (double)Ih.y + (double)Il.y);
+    const int j3 = j3_0 + 2 * h;
+    double2 *o = RAG ? partial + (long long)chunk * NN * N + (j1 * N + j2) * N + j3
+                     : partial + (long long)chunk * NN * N + kcol + 2 * h;
+    if (!RAG || j3 < N)
+      o[0] = make_double2((double)Rh.x + (double)Rl.x, (double)Ih.x + (double)Il.x);
+    if (!RAG || j3 + 1 < N)
+      o[1] = make_double2((double)Rh.y + (double)Rl.y, (double)Ih.y + (double)Il.y);
   }
 }
 
@@ -770,46 +756,49 @@ struct C64pShape {
 };
 constexpr C64pShape kC64pShapes[] = {{256, 2, 4}, {256, 2, 2}, {128, 3, 2}, {128, 4, 2}, {256, 2, 1}};
 static_assert(sizeof(kC64pShapes) / sizeof(kC64pShapes[0]) == kC64xNShapes, "shape count");
-// the output-pair kernel runs the pair table when N is a multiple of 4
-static bool c64_op(const QParams &p, bool paired) { return paired && p.N % RUN == 0; }
-
-// N fixed at compile time for the output-pair kernel's tensor-copy form from
-// N = 20 up (0: runtime N): N = 20 109 -> 105 us, N = 28 629 -> 605 us per sum;
-// at N = 16 40.3 us either way.
-static int c64_nc(const QParams &p, bool op, bool tma) {
-  return (op && tma && p.N >= 20 && p.N <= 32) ? p.N : 0;
-}
-template <bool TMA, int S>
-static const void *c64x_fn_s(bool op, int nc) {
+// The output-pair kernel of a shape.  N fixed at compile time from N = 20 up in
+// fours: N = 20 109 -> 105 us, N = 28 629 -> 605 us per sum; at N = 16 40.3 us
+// either way.
+typedef void (*C64pFn)(QParams, int, int, const float4 *, double2 *, unsigned long long,
+                       const CUtensorMap);
+template <int S>
+static C64pFn c64p_fn_s(int N) {
   constexpr int T = kC64pShapes[S].maxt, B = kC64pShapes[S].minb, R = kC64pShapes[S].rows;
-  if (op) {
-    if constexpr (TMA) {
-      if (nc == 20) return (const void *)calq64p_kernel<TMA, T, B, R, 20>;
-      if (nc == 24) return (const void *)calq64p_kernel<TMA, T, B, R, 24>;
-      if (nc == 28) return (const void *)calq64p_kernel<TMA, T, B, R, 28>;
-      if (nc == 32) return (const void *)calq64p_kernel<TMA, T, B, R, 32>;
-    }
-    return (const void *)calq64p_kernel<TMA, T, B, R, 0>;
-  }
-  return (const void *)calq64x_kernel<TMA, kC64xShapes[S].maxt, kC64xShapes[S].minb>;
+  if (N % RUN) return calq64p_kernel<T, B, R, 0, true>;
+  if (N == 20) return calq64p_kernel<T, B, R, 20, false>;
+  if (N == 24) return calq64p_kernel<T, B, R, 24, false>;
+  if (N == 28) return calq64p_kernel<T, B, R, 28, false>;
+  if (N == 32) return calq64p_kernel<T, B, R, 32, false>;
+  return calq64p_kernel<T, B, R, 0, false>;
 }
-template <bool TMA>
-static const void *c64x_fn(int shape, bool op, int nc) {
+static C64pFn c64p_fn(int shape, int N) {
   switch (shape) {
-    case 0: return c64x_fn_s<TMA, 0>(op, nc);
-    case 1: return c64x_fn_s<TMA, 1>(op, nc);
-    case 2: return c64x_fn_s<TMA, 2>(op, nc);
-    case 3: return c64x_fn_s<TMA, 3>(op, nc);
-    default: return c64x_fn_s<TMA, 4>(op, nc);
+    case 0: return c64p_fn_s<0>(N);
+    case 1: return c64p_fn_s<1>(N);
+    case 2: return c64p_fn_s<2>(N);
+    case 3: return c64p_fn_s<3>(N);
+    default: return c64p_fn_s<4>(N);
+  }
+}
+typedef void (*C64xFn)(QParams, int, int, const float2 *, const float4 *, double2 *,
+                       unsigned long long);
+template <bool TMA>
+static C64xFn c64x_fn(int shape) {
+  switch (shape) {
+    case 0: return calq64x_kernel<TMA, kC64xShapes[0].maxt, kC64xShapes[0].minb>;
+    case 1: return calq64x_kernel<TMA, kC64xShapes[1].maxt, kC64xShapes[1].minb>;
+    case 2: return calq64x_kernel<TMA, kC64xShapes[2].maxt, kC64xShapes[2].minb>;
+    case 3: return calq64x_kernel<TMA, kC64xShapes[3].maxt, kC64xShapes[3].minb>;
+    default: return calq64x_kernel<TMA, kC64xShapes[4].maxt, kC64xShapes[4].minb>;
   }
 }
 
 static size_t c64x_smem(int N, int threads, bool tma, bool op, int rows) {
   const int nwarps = (threads + 31) / 32;
   if (op) {
-    size_t o = (size_t)nwarps * (PDEPTH / rows) * 8;
-    if (tma) o += 2 * sizeof(float4) * (size_t)nwarps * PDEPTH * std::min(32, threads);
-    return o + 2 * sizeof(float4) * (size_t)N * N;
+    return (size_t)nwarps * (PDEPTH / rows) * 8 +
+           2 * sizeof(float4) * (size_t)nwarps * PDEPTH * p64_box_threads(threads) +
+           2 * sizeof(float4) * (size_t)N * ((N + RUN - 1) / RUN * RUN);
   }
   size_t o = 16 * (size_t)((nwarps * DEPTH * 8 + 15) / 16);
   if (tma) o += sizeof(float2) * (size_t)nwarps * DEPTH * 32 * RUN;
@@ -851,7 +840,7 @@ static C64xPlan c64x_plan_compute(const QParams &p, bool aligned, int shape_in, 
   C64xPlan pl;
   const int shape = shape_in % kC64xNShapes;
   const bool model = shape_in >= kC64xNShapes;
-  const bool op = c64_op(p, paired);
+  const bool op = paired;
   const int R4 = (p.P + RUN - 1) / RUN;
   int J2T = std::max(1, (op ? kC64pShapes[shape].maxt : kC64xShapes[shape].maxt) / R4);
   if (J2T > p.P) J2T = p.P;
@@ -860,11 +849,12 @@ static C64xPlan c64x_plan_compute(const QParams &p, bool aligned, int shape_in, 
   pl.J2T = J2T;
   pl.tiles = tiles;
   pl.threads = J2T * R4;
-  pl.tma = aligned && (p.P % RUN) == 0 && (p.P % J2T) == 0;
+  pl.tma = op || (aligned && (p.P % RUN) == 0 && (p.P % J2T) == 0);
   pl.smem = c64x_smem(p.N, pl.threads, pl.tma, op, kC64pShapes[shape].rows);
   int occ = 1;
-  const int nc = c64_nc(p, op, pl.tma);
-  const void *fn = pl.tma ? c64x_fn<true>(shape, op, nc) : c64x_fn<false>(shape, op, nc);
+  const void *fn = op       ? (const void *)c64p_fn(shape, p.N)
+                   : pl.tma ? (const void *)c64x_fn<true>(shape)
+                            : (const void *)c64x_fn<false>(shape);
   cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, pl.threads, pl.smem);
   if (occ < 1) occ = 1;
@@ -951,8 +941,13 @@ edb_status launch_split_B(long long n, const double *B, float2 *B2, cudaStream_t
   return EDB_OK;
 }
 
+long long calq64x_table(int N, bool paired) {
+  const long long NQ = (long long)N * N * N;
+  return NQ * (paired ? (long long)N * N * ((N + RUN - 1) / RUN * RUN) : NQ);
+}
+
 edb_status launch_split_B_paired(int N, const double *B, float2 *B2, cudaStream_t st) {
-  const long long n = (long long)N * N * N * N * N * N;
+  const long long n = calq64x_table(N, true);
   b2_pair_split_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(N, B, B2);
   EDB_LAUNCHED();
   return EDB_OK;
@@ -960,72 +955,37 @@ edb_status launch_split_B_paired(int N, const double *B, float2 *B2, cudaStream_
 
 int calq64x_shapes() { return 2 * kC64xNShapes; }
 
-template <bool TMA, int S>
-static void c64x_launch_s(dim3 grid, const C64xPlan &pl, const QParams &p, bool paired,
-                          const float2 *d_B2, const float4 *d_fdf, double2 *d_partial,
-                          const CUtensorMap &tm, cudaStream_t st) {
-  constexpr int T = kC64pShapes[S].maxt, B = kC64pShapes[S].minb, R = kC64pShapes[S].rows;
-  const float4 *B2p = reinterpret_cast<const float4 *>(d_B2);
-  if (c64_op(p, paired)) {
-    const int nc = c64_nc(p, true, TMA);
-    auto *fn = calq64p_kernel<TMA, T, B, R, 0>;
-    if constexpr (TMA) {
-      if (nc == 20) fn = calq64p_kernel<TMA, T, B, R, 20>;
-      if (nc == 24) fn = calq64p_kernel<TMA, T, B, R, 24>;
-      if (nc == 28) fn = calq64p_kernel<TMA, T, B, R, 28>;
-      if (nc == 32) fn = calq64p_kernel<TMA, T, B, R, 32>;
-    }
-    fn<<<grid, pl.threads, pl.smem, st>>>(p, pl.J2T, pl.LC, B2p, d_fdf, d_partial,
-                                          wait_limit_ns(), tm);
-  } else
-    calq64x_kernel<TMA, kC64xShapes[S].maxt, kC64xShapes[S].minb>
-        <<<grid, pl.threads, pl.smem, st>>>(p, pl.J2T, pl.LC, paired, d_B2, d_fdf, d_partial,
-                                            wait_limit_ns());
-}
-template <bool TMA>
-static void c64x_launch(int shape, dim3 grid, const C64xPlan &pl, const QParams &p, bool paired,
-                        const float2 *d_B2, const float4 *d_fdf, double2 *d_partial,
-                        const CUtensorMap &tm, cudaStream_t st) {
-  switch (shape) {
-    case 0: c64x_launch_s<TMA, 0>(grid, pl, p, paired, d_B2, d_fdf, d_partial, tm, st); break;
-    case 1: c64x_launch_s<TMA, 1>(grid, pl, p, paired, d_B2, d_fdf, d_partial, tm, st); break;
-    case 2: c64x_launch_s<TMA, 2>(grid, pl, p, paired, d_B2, d_fdf, d_partial, tm, st); break;
-    case 3: c64x_launch_s<TMA, 3>(grid, pl, p, paired, d_B2, d_fdf, d_partial, tm, st); break;
-    default: c64x_launch_s<TMA, 4>(grid, pl, p, paired, d_B2, d_fdf, d_partial, tm, st); break;
-  }
-}
-
 edb_status launch_calq64x(const QParams &p, const float2 *d_B2, const double2 *d_in,
                           float4 *d_fdf, double2 *d_partial, double2 *d_Q, cudaStream_t st,
                           int shape, bool paired) {
   if (shape < 0 || shape >= 2 * kC64xNShapes) shape = 0;
   if (paired && (p.P != p.N || (p.sM % p.N) != 0 || (p.sL % p.N) != p.N - p.n))
     return fail(EDB_EINVAL, "calq64x: pairs need the aliased index shifts");
-  if (c64_op(p, paired)) {
-    fdr_split_kernel<<<(unsigned)((p.NQ + 1 + 255) / 256), 256, 0, st>>>(p.N, p.sL % p.N, d_in,
-                                                                        d_fdf);
-  } else {
-    fdf_split_kernel<<<(unsigned)((p.NQ + 255) / 256), 256, 0, st>>>(p.NQ, d_in, d_fdf);
-  }
-  EDB_LAUNCHED();
   const bool aligned = ((uintptr_t)d_B2 % 16) == 0;
-  if (c64_op(p, paired) && !aligned)
+  if (paired && !aligned)
     return fail(EDB_EINVAL, "calq64x: the output-pair table must be 16-byte aligned");
   const C64xPlan pl = c64x_plan(p, aligned, shape, paired);
-  dim3 grid((unsigned)p.P, (unsigned)pl.tiles, (unsigned)pl.nch);
-  CUtensorMap tm = {};
-  if (pl.tma && c64_op(p, paired)) {
-    const cuuint64_t dim[2] = {(cuuint64_t)(2 * p.NQ), (cuuint64_t)p.NQ};
-    const cuuint64_t str[1] = {(cuuint64_t)(8 * p.NQ)};
-    const cuuint32_t box[2] = {(cuuint32_t)(8 * std::min(32, pl.threads)),
-                               (cuuint32_t)kC64pShapes[shape % kC64xNShapes].rows};
+  const dim3 grid((unsigned)p.P, (unsigned)pl.tiles, (unsigned)pl.nch);
+  const int s = shape % kC64xNShapes;
+  if (paired) {
+    CUtensorMap tm;
+    const cuuint64_t dim[2] = {(cuuint64_t)(2 * calq64x_table(p.N, true) / p.NQ), (cuuint64_t)p.NQ};
+    const cuuint64_t str[1] = {4 * dim[0]};
+    const cuuint32_t box[2] = {(cuuint32_t)(8 * p64_box_threads(pl.threads)),
+                               (cuuint32_t)kC64pShapes[s].rows};
     if (!encode_map(&tm, 2, d_B2, dim, str, box))
       return fail(EDB_ECUDA, "calq64x: cuTensorMapEncodeTiled");
+    fdr_split_kernel<<<(unsigned)((p.NQ + 1 + 255) / 256), 256, 0, st>>>(p.N, p.sL % p.N, d_in,
+                                                                        d_fdf);
+    EDB_LAUNCHED();
+    c64p_fn(s, p.N)<<<grid, pl.threads, pl.smem, st>>>(p, pl.J2T, pl.LC, d_fdf, d_partial,
+                                                       wait_limit_ns(), tm);
+  } else {
+    fdf_split_kernel<<<(unsigned)((p.NQ + 255) / 256), 256, 0, st>>>(p.NQ, d_in, d_fdf);
+    EDB_LAUNCHED();
+    (pl.tma ? c64x_fn<true>(s) : c64x_fn<false>(s))<<<grid, pl.threads, pl.smem, st>>>(
+        p, pl.J2T, pl.LC, d_B2, d_fdf, d_partial, wait_limit_ns());
   }
-  if (pl.tma)
-    c64x_launch<true>(shape % kC64xNShapes, grid, pl, p, paired, d_B2, d_fdf, d_partial, tm, st);
-  else
-    c64x_launch<false>(shape % kC64xNShapes, grid, pl, p, paired, d_B2, d_fdf, d_partial, tm, st);
   EDB_LAUNCHED();
   return launch_calq64_reduce(p, pl.nch, d_partial, d_Q, st);
 }

@@ -1,7 +1,8 @@
-"""The table copies of the double-float sum at N % 4 == 0.
+"""The table copies of the double-float sum over pairs.
 
-Sizes: CTAs of under one warp (N = 4, 8), with a last warp that is partly empty
-(N = 12, 20, 24, 28) and of full warps (N = 16); every launch shape, so every
+Sizes: CTAs of under one warp (N = 3, 4, 6, 8), with a last warp that is partly
+empty (N = 12, 20, 24, 28) and of full warps (N = 16); rows padded by one, two and
+three entries (N = 3, 7 | 6, 18, 30 | 9, 17, 25); every launch shape, so every
 number of rows a copy, and both rules for the l-line chunks.
 
 Tolerance: the drop-in path's bound, relative L2 <= 1e-12.
@@ -21,7 +22,7 @@ def edb():
     return e
 
 
-@pytest.mark.parametrize("N", [4, 8, 12, 16, 20, 24, 28])
+@pytest.mark.parametrize("N", [3, 4, 6, 7, 8, 9, 12, 16, 17, 18, 20, 24, 25, 28, 30])
 def test_every_launch_shape_against_the_direct_sum(edb, oracle, N):
     L = 6.0
     rng = np.random.default_rng(N)
