@@ -1409,6 +1409,16 @@ constexpr C32Variant kC32Variants[] = {
 int calq32_variants() { return (int)(sizeof(kC32Variants) / sizeof(kC32Variants[0])); }
 int calq32_group(int variant) { return kC32Variants[variant].sc * kC32Variants[variant].ws; }
 bool calq32_pair(int variant) { return kC32Variants[variant].pair; }
+bool calq32_one_solve(int variant) { return kC32Variants[variant].sc == 1; }
+// Under 16 solves the other variants leave solve lanes empty, and above that
+// they may leave SMs without a CTA (16 x N = 16, 16 work items: 102 us against
+// 191); with both filled they need twice the shared-memory reads, and timing
+// them only delays a new state's first step.
+bool calq32_few(int N, int S, int C) {
+  if (S < 16) return true;
+  const int K2T = std::max(1, std::min(N, 256 / (8 * ((N + 7) / 8))));  // variant 0's tile
+  return (long long)((S + 15) / 16) * C * N * ((N + K2T - 1) / K2T) < device_sm_count();
+}
 size_t calq32_pair_bytes(int N, int S) { return (size_t)((S + 1) / 2) * N * N * N * sizeof(float4); }
 
 // Tensor maps of one launch (tmap = 0: bulk copies, the maps are unused).
