@@ -558,9 +558,8 @@ extern "C" edb_status edb_qcalc_calQ_batch_f32_device(edb_qcalc *q, int S, const
 // Times every variant of the batched kernel on the caller's buffers (chunk
 // count C, partial buffer for C > 1; one launch each behind a warm-up that
 // hides its host side, CUDA events on `st`) and records the fastest for S's
-// class.  The pair variants take part when the caller passes a pair buffer, the
-// one-solve variants where they can win (calq32_few).  Two timed launches chose
-// no better and made a new state wait longer: 128 x N = 24 101 -> 71 ms before
+// class.  The pair variants take part when the caller passes a pair buffer.  Two
+// timed launches chose no better and made a new state wait longer: 128 x N = 24 101 -> 71 ms before
 // its first step, 256 cells x N = 16 20 -> 14 ms.
 static edb_status autotune_c32(edb_qcalc *q, int S, const float2 *d_fin, float2 *d_Qout,
                                cudaStream_t st, int C, float4 *d_partial, float4 *d_pairs,
@@ -579,7 +578,6 @@ static edb_status autotune_c32(edb_qcalc *q, int S, const float2 *d_fin, float2 
   for (int v = 0; v < calq32_variants() && rc == EDB_OK; ++v) {
     if (calq32_pair(v) && !d_pairs) continue;
     if (calq32_group(v) < 16 && S > 64) continue;  // small groups are for few solves
-    if (calq32_one_solve(v) && !calq32_few(q->d.N, S, C)) continue;
     rc = launch_calq32_batch(q->d.N, S, q->B32, d_fin, d_Qout, st, v, C, d_partial, d_pairs,
                              persist);
     if (rc == EDB_EINVAL) {  // this variant does not fit this N: skip it

@@ -202,9 +202,6 @@ edb_status calq32_status_ptr(int **p);
 int calq32_variants();
 int calq32_group(int variant);  // solves per CTA group
 bool calq32_pair(int variant);
-bool calq32_one_solve(int variant);
-// Whether the one-solve variants can be the fastest for S solves in C chunks.
-bool calq32_few(int N, int S, int C);
 size_t calq32_pair_bytes(int N, int S);
 // persist: run the plain-layout, tensor-copy launches as one persistent grid.
 // -1: only without chunks, where it is faster alone, with the CTA work items

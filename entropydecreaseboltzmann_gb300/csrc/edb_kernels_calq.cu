@@ -1388,8 +1388,8 @@ __global__ void calq32_reduce_kernel(long long n, int C, const float4 *__restric
 //   11: WS 2, the same (2-solve groups)
 //   12, 13: 10 and 11 with stages kept small enough for one wave of CTAs
 // 10-13 are for the few solves that leave 16-solve lanes empty.  us without
-// chunks, best of 0-9 -> best of 10-13: 4 x N = 16 191 -> 95, 4 x N = 24 718 -> 244,
-// 4 x N = 32 2100 -> 1000; in 4 chunks 76 -> 49, 296 -> 224, 2126 -> 760.
+// chunks, best of 0-9 -> best of 10-13: 4 x N = 16 191 -> 96, 4 x N = 24 646 -> 266,
+// 4 x N = 32 2096 -> 1101, 18 x N = 32 3209 -> 2998; in 4 chunks 76 -> 49, 296 -> 224, 2126 -> 760.
 struct C32Variant {
   int ws, a, maxt;
   bool hls;
@@ -1409,16 +1409,6 @@ constexpr C32Variant kC32Variants[] = {
 int calq32_variants() { return (int)(sizeof(kC32Variants) / sizeof(kC32Variants[0])); }
 int calq32_group(int variant) { return kC32Variants[variant].sc * kC32Variants[variant].ws; }
 bool calq32_pair(int variant) { return kC32Variants[variant].pair; }
-bool calq32_one_solve(int variant) { return kC32Variants[variant].sc == 1; }
-// Under 16 solves the other variants leave solve lanes empty, and above that
-// they may leave SMs without a CTA (16 x N = 16, 16 work items: 102 us against
-// 191); with both filled they need twice the shared-memory reads, and timing
-// them only delays a new state's first step.
-bool calq32_few(int N, int S, int C) {
-  if (S < 16) return true;
-  const int K2T = std::max(1, std::min(N, 256 / (8 * ((N + 7) / 8))));  // variant 0's tile
-  return (long long)((S + 15) / 16) * C * N * ((N + K2T - 1) / K2T) < device_sm_count();
-}
 size_t calq32_pair_bytes(int N, int S) { return (size_t)((S + 1) / 2) * N * N * N * sizeof(float4); }
 
 // Tensor maps of one launch (tmap = 0: bulk copies, the maps are unused).
@@ -1614,6 +1604,29 @@ static edb_status launch_c32_reduce(int N, int S, int C, const float4 *d_partial
   return EDB_OK;
 }
 
+// The solves of a last, at most half full group of 16 that are worth a launch
+// of one-solve variant 10 to themselves (0: none): those whose group starts a
+// new wave of CTAs.  A wave costs what its fullest CTA does, the remainder's own
+// launch 0.4 to 0.55 of that up to four solves and 0.75 up to eight, which pays
+// from four full groups on.  33 x N = 24 1203 -> 986 us, 66 2076 -> 1695, 130
+// 3390 -> 3060, 72 2077 -> 1954; 130 x N = 32 16.12 -> 15.29 ms; where no wave is
+// saved (130 x N = 16 301 us) the remainder stays with the rest.
+static int c32_remainder(int N, int S, const C32Variant &vr, const float *d_B32,
+                         const float2 *d_fin) {
+  const int SG = vr.sc * vr.ws, r = S % 16;
+  if (vr.pair || SG != 16 || S < 16 || r < 1 || r > (S < 64 ? 4 : 8)) return 0;
+  long long waves[2];
+  const long long slots = (long long)device_sm_count() * vr.minb;
+  for (int i = 0; i < 2; ++i) {
+    C32Setup su;
+    const int s = i ? S - r : S;
+    if (c32_setup(N, s, vr, 1, d_B32, d_fin, 0, &su) != EDB_OK || !su.tma || !su.maps.tmap)
+      return 0;
+    waves[i] = ((long long)((s + 15) / 16) * N * su.tiles + slots - 1) / slots;
+  }
+  return waves[0] > waves[1] ? r : 0;
+}
+
 edb_status launch_calq32_batch(int N, int S, const float *d_B32, const float2 *d_fin, float2 *d_Q,
                                cudaStream_t st, int variant, int C, float4 *d_partial,
                                float4 *d_pairs, int persist) {
@@ -1634,6 +1647,16 @@ edb_status launch_calq32_batch(int N, int S, const float *d_B32, const float2 *d
   }
   const C32Variant &vr = kC32Variants[variant];
   if (vr.pair && !d_pairs) return fail(EDB_EINVAL, "calq32: pair variants need a pair buffer");
+  if (C == 1) {
+    const int r = c32_remainder(N, S, vr, d_B32, d_fin);
+    if (r) {
+      const size_t at = (size_t)(S - r) * N * N * N;
+      EDB_TRY(launch_calq32_batch(N, S - r, d_B32, d_fin, d_Q, st, variant, 1, nullptr, d_pairs,
+                                  persist));
+      return launch_calq32_batch(N, r, d_B32, d_fin + at, d_Q + at, st, 10, 1, nullptr, nullptr,
+                                 persist);
+    }
+  }
   const int SG = vr.sc * vr.ws;
   const float2 *src = vr.pair ? reinterpret_cast<const float2 *>(d_pairs) : d_fin;
   C32Setup su;
