@@ -41,7 +41,7 @@
 // What bounds it: the instruction issue of the hand-overs and of the A rows
 // beside the FMAs (a tile of N = 24 takes about 240 clocks an SM, its FMAs 60).
 // Measured, ms: 37 solves of N = 21 2.80 (calq32_kernel's plain-load path) ->
-// 0.95, 256 of N = 31 126 -> 31, 16 of N = 17 0.82 -> 0.16.
+// 0.80, 256 of N = 31 126 -> 31, 16 of N = 17 0.82 -> 0.16.
 #include <algorithm>
 
 #include "edb_internal.cuh"
@@ -313,6 +313,7 @@ TcGeom tc_geom(int N) {
 
 struct TcArgs {
   int N, S, CL, V, pitch, C, NST, FL;  // FL: steps per fold
+  int first, end;                      // this launch's solves
   const float *B32;
   const float2 *fin;
   float2 *Q;
@@ -389,12 +390,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1) calqtc_kernel(const TcArgs a) {
 
   // CTA -> (solve group, k1, chunk): groups fastest, so that the CTAs in
   // flight read the same weights at about the same time
-  const int groups = (a.S + SG - 1) / SG;
+  const int groups = (a.end - a.first + SG - 1) / SG;
   const int grp = blockIdx.x % groups;
   const int rest = blockIdx.x / groups;
   const int chunk = rest % C, k1 = rest / C;
-  const int s0 = grp * SG;
-  const int ns = min(SG, a.S - s0);
+  const int s0 = a.first + grp * SG;
+  const int ns = min(SG, a.end - s0);
   const int nlist = c32_nlist(N, k1), plo = k1 / 2;
   const int ppc = (nlist + C - 1) / C;
   const int P0 = min(nlist, chunk * ppc), np = min(nlist, P0 + ppc) - P0;
@@ -828,9 +829,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1) calqtc_kernel(const TcArgs a) {
 }
 
 template <int NC, int SG>
-static edb_status launch_tc(const TcArgs &args, cudaStream_t st) {
+static edb_status launch_tc(const TcArgs &args, int first, int end, cudaStream_t st) {
   using Cfg = TcCfg<NC, SG>;
+  if (first >= end) return EDB_OK;
   TcArgs a = args;
+  a.first = first;
+  a.end = end;
   auto kern = calqtc_kernel<NC, SG>;
   static const cudaError_t configured =
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
@@ -842,7 +846,7 @@ static edb_status launch_tc(const TcArgs &args, cudaStream_t st) {
   // at least half of an SM's shared memory: one CTA per SM holds all of its
   // tensor memory
   const size_t bytes = std::max<size_t>(fixed + (size_t)a.NST * Cfg::SB, 120 * 1024);
-  const long long blocks = (long long)((a.S + SG - 1) / SG) * a.N * a.C;
+  const long long blocks = (long long)((end - first + SG - 1) / SG) * a.N * a.C;
   kern<<<(unsigned)blocks, TC_THREADS, bytes, st>>>(a);
   EDB_LAUNCHED();
   return EDB_OK;
@@ -866,10 +870,31 @@ edb_status launch_calqtc(int N, int S, const float *d_B32, const float2 *d_fin, 
   a.wait_ns = wait_limit_ns();
   EDB_TRY(calq32_status_ptr(&a.status));
   a.NST = 0;
-  // solves per CTA: 4, or 2 where 4 would leave half of the SMs idle
-  const int SG = (long long)((S + 3) / 4) * N * C * 2 <= device_sm_count() ? 2 : 4;
-#define EDB_TC(NC) \
-  return SG == 4 ? launch_tc<NC, 4>(a, st) : launch_tc<NC, 2>(a, st)
+  // Solves per CTA: 4 for the first `four` solves and 2 for the others, in a
+  // launch of their own, by the number of CTA waves.  A wave of CTAs of 2 takes
+  // 0.67 of one of 4 at 16 weight columns and 0.63 above (N = 13 74 | 109 us, 21
+  // 311 | 492, 31 1476 | 2285): 37 x N = 21 944 us in CTAs of 4 (210 of them on 152
+  // SMs), 887 in CTAs of 2, 795 as 28 + 9; 17 x N = 31 4.44 -> 2.86 ms, 30 x N = 25
+  // 1.90 -> 1.59 ms.  A second launch has to gain 3% and its start: over many waves
+  // the CTAs drift apart, and a last one that is part full costs less (500 x N = 21
+  // 8.45 ms, 8.55 as 492 + 8).
+  const long long per = (long long)N * C, sms = device_sm_count();
+  auto waves = [&](long long groups) { return (double)((groups * per + sms - 1) / sms); };
+  const int all = (S + 3) / 4;
+  int four = S;
+  double best = 1e30;
+  for (int g4 = all; g4 >= 0; --g4) {
+    const int n4 = std::min(S, 4 * g4), n2 = S - n4;
+    double t = waves(g4) + (g.NC == 16 ? 0.67 : 0.63) * waves((n2 + 1) / 2);
+    if (n2 > 0 && n4 > 0) t = 1.03 * t + 0.02;
+    if (t < best - 1e-9) {
+      best = t;
+      four = n4;
+    }
+  }
+#define EDB_TC(NC)                                \
+  EDB_TRY((launch_tc<NC, 4>(a, 0, four, st)));    \
+  return launch_tc<NC, 2>(a, four, S, st)
   switch (g.NC) {
     case 16: EDB_TC(16);
     case 24: EDB_TC(24);

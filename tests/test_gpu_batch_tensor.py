@@ -101,3 +101,24 @@ def test_wait_timeout_is_reported_and_recovers(edb):
     torch.cuda.synchronize()
     assert edb.device_status(clear=True) == 0
     assert torch.equal(again, good)
+
+
+@pytest.mark.parametrize("N,S", [(13, 50), (21, 37), (25, 31), (31, 17)])
+def test_a_batch_in_two_launches_has_each_solves_own_bits(N, S):
+    """Sizes whose solves go part in CTAs of four and part in CTAs of two; chunks
+    keep their place in the caller's partial sums."""
+    import torch
+    import entropydecreaseboltzmann_gb300 as edb
+
+    _, fin = _inputs(N, S, seed=N)
+    q = edb.QCalculator(N, 0, gamma=0.0, L=6.0, filter=False, index_mode=INDEX_ALIASED)
+    q.genB()
+    for chunks in (1, 3):
+        part = torch.empty(chunks * S * N ** 3 * 4, dtype=torch.float32, device="cuda")
+        out = torch.full_like(fin, float("nan"))
+        q.calQ_batch_f32_ex(S, 0, chunks, part, fin, out)
+        for s in range(S):
+            one = torch.empty_like(fin[:1])
+            q.calQ_batch_f32_ex(1, 0, chunks, part, fin[s:s + 1], one)
+            assert torch.equal(one, out[s:s + 1]), (chunks, s)
+    assert edb.device_status() == 0
