@@ -120,8 +120,40 @@ int calq64_nchunk(const QParams &p);
 edb_status launch_calq64(const QParams &p, const double *d_B, const double2 *d_fin,
                          double2 *d_partial, double2 *d_Q, cudaStream_t st);
 
+// early: started before its predecessor on the stream has ended (launch_early).
 edb_status launch_calq64_reduce(const QParams &p, int nchunk, const double2 *d_partial,
-                                double2 *d_Q, cudaStream_t st);
+                                double2 *d_Q, cudaStream_t st, bool early = false);
+
+// A kernel whose blocks may start once every block of the kernel before it on
+// the stream has called dep_launch() or ended; before it reads what that kernel writes,
+// or writes anything that kernel reads, each of its threads calls dep_wait(),
+// which returns when that kernel has ended and its writes are visible.  Such
+// data is read by plain loads: the read-only path may not see it.
+template <typename... P, typename... A>
+inline edb_status launch_early(void (*fn)(P...), dim3 grid, int threads, size_t smem,
+                               cudaStream_t st, A &&...args) {
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  EDB_CUDA(cudaLaunchKernelEx(&cfg, fn, static_cast<P>(args)...));
+  count_launch();
+  return EDB_OK;
+}
+#ifdef __CUDACC__
+__device__ __forceinline__ void dep_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void dep_launch() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+#endif
 
 // FP64-accurate calQ on the FP32 pipe (double-float arithmetic): B2 is the
 // table split into (hi, lo) floats, fdf (N^3 float4) the input split into

@@ -113,8 +113,8 @@ __global__ void __launch_bounds__(CALQ64_THREADS)
 // took 51.3 us, the N = 12 sum 35.4.
 constexpr int RED_PARTS = 4, RED_OUT = 32 / RED_PARTS, RED_WARPS = 4, RED_AHEAD = 8;
 __global__ void __launch_bounds__(32 * RED_WARPS)
-    calq64_reduce_kernel(QParams p, int nchunk, const double2 *__restrict__ partial,
-                         double2 *__restrict__ Q) {
+    calq64_reduce_kernel(QParams p, int nchunk, const double2 *partial, double2 *Q) {
+  dep_wait();
   const int N = p.N, n = p.n;
   const int lane = threadIdx.x & 31, part = lane / RED_OUT;
   const long long k =
@@ -182,7 +182,10 @@ edb_status launch_calq64(const QParams &p, const double *d_B, const double2 *d_f
 // double-float kernel (edb_kernels_calq64x.cu), which writes the same partial
 // layout.
 edb_status launch_calq64_reduce(const QParams &p, int nchunk, const double2 *d_partial,
-                                double2 *d_Q, cudaStream_t st) {
+                                double2 *d_Q, cudaStream_t st, bool early) {
+  if (early)
+    return launch_early(calq64_reduce_kernel, dim3(red_blocks(p.NQ)), 32 * RED_WARPS, 0, st, p,
+                        nchunk, d_partial, d_Q);
   calq64_reduce_kernel<<<red_blocks(p.NQ), 32 * RED_WARPS, 0, st>>>(p, nchunk, d_partial, d_Q);
   EDB_LAUNCHED();
   return EDB_OK;

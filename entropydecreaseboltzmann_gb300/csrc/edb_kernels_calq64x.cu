@@ -478,6 +478,11 @@ __global__ void __launch_bounds__(MAXT, MINB)
 // error against the FP64 kernel on near-equilibrium data, that form -> folded
 // (unfolded): N = 9 1.7e-14 -> 2.2e-14 (3.0e-14), 17 5.0e-14 -> 2.6e-14 (8.6e-14),
 // 23 9.1e-14 -> 3.6e-14 (1.6e-13), 30 6.7e-13 -> 6.8e-14 (6.5e-13).
+// Launches: the kernel starts as the split of f-hat ends (its own start and the
+// first table rows run under that kernel's end), and the reduction as this one
+// ends: N = 8 20.6 -> 14.4 us a sum, 12 27.8 -> 22.6, 16 40.4 -> 35.1, 17 69.7 ->
+// 65.5, 24 262.0 -> 257.5, 32 1052 -> 1050.  Its blocks do not come before the
+// split's are done (an early trigger there left some SMs a block short).
 constexpr int PDEPTH = 8;
 // Threads whose entries one ring row holds: a warp's, or all of a CTA of under
 // one warp (N < 12), in fours so that a slot starts on a 128-byte boundary.
@@ -496,7 +501,7 @@ __host__ __device__ constexpr int p64_box_threads(int threads) {
 // past its own are other threads' and are not read).
 template <int MAXT, int MINB, int ROWS, int NC, bool RAG>
 __global__ void __launch_bounds__(MAXT, MINB)
-    calq64p_kernel(QParams p, int J2T, int LC, const float4 *__restrict__ fdr, double2 *__restrict__ partial,
+    calq64p_kernel(QParams p, int J2T, int LC, const float4 *fdr, double2 *partial,
                    unsigned long long wait_ns, const __grid_constant__ CUtensorMap tmB) {
   constexpr int SLOTS = PDEPTH / ROWS;
   static_assert(SLOTS * ROWS == PDEPTH && RUN % ROWS == 0, "ring shape");
@@ -584,6 +589,8 @@ __global__ void __launch_bounds__(MAXT, MINB)
   }
   __syncwarp(wmask);
   for (int sl = 0; sl < SLOTS; ++sl) refill(sl, true);  // rows [0, PDEPTH)
+  // the table's first rows are on their way; f-hat's split may still be written
+  dep_wait();
 
   DF2 accR[2], accI[2];  // lanes (j3_0 + 2h, j3_0 + 2h + 1)
 #pragma unroll
@@ -641,7 +648,7 @@ __global__ void __launch_bounds__(MAXT, MINB)
       load_e(2 * R4 + r, 2);  // x = 4r + 2: E[x + 2] of step 0 = the entry of step -2
     }
     int x = j3_0;
-    float4 fl_next = __ldg(flp);
+    float4 fl_next = *flp;
     int am = r;
     // at N = 24 two groups per iteration (0.304 -> 0.298 ms per launch); at
     // N = 32 that measured 1% slower
@@ -670,7 +677,7 @@ __global__ void __launch_bounds__(MAXT, MINB)
           load_e((4 - t) * R4 + an, t);
         }
         const float4 fl = fl_next;
-        fl_next = __ldg(flp + g + t + 1);
+        fl_next = flp[g + t + 1];
         const u64 xr = pk(fl.x, fl.x), nxr = pk(-fl.x, -fl.x), nlr = pk(-fl.z, -fl.z);
         const u64 xi = pk(fl.y, fl.y), nxi = pk(-fl.y, -fl.y), nli = pk(-fl.w, -fl.w);
         const u64 li = pk(fl.w, fl.w);
@@ -701,6 +708,9 @@ __global__ void __launch_bounds__(MAXT, MINB)
       am = an;
     }
   }
+  // the reduction's blocks may come in (from the start on they took slots that
+  // this kernel's last blocks wanted: N = 16 43 us against 35)
+  dep_launch();
   if (__syncthreads_or(to)) {
     if (lane == 0) {
       atomicExch(&g_calq64x_status, 1);
@@ -978,16 +988,16 @@ edb_status launch_calq64x(const QParams &p, const float2 *d_B2, const double2 *d
     fdr_split_kernel<<<(unsigned)((p.NQ + 1 + 255) / 256), 256, 0, st>>>(p.N, p.sL % p.N, d_in,
                                                                         d_fdf);
     EDB_LAUNCHED();
-    c64p_fn(s, p.N)<<<grid, pl.threads, pl.smem, st>>>(p, pl.J2T, pl.LC, d_fdf, d_partial,
-                                                       wait_limit_ns(), tm);
+    EDB_TRY(launch_early(c64p_fn(s, p.N), grid, pl.threads, pl.smem, st, p, pl.J2T, pl.LC, d_fdf,
+                         d_partial, wait_limit_ns(), tm));
   } else {
     fdf_split_kernel<<<(unsigned)((p.NQ + 255) / 256), 256, 0, st>>>(p.NQ, d_in, d_fdf);
     EDB_LAUNCHED();
     (pl.tma ? c64x_fn<true>(s) : c64x_fn<false>(s))<<<grid, pl.threads, pl.smem, st>>>(
         p, pl.J2T, pl.LC, d_B2, d_fdf, d_partial, wait_limit_ns());
+    EDB_LAUNCHED();
   }
-  EDB_LAUNCHED();
-  return launch_calq64_reduce(p, pl.nch, d_partial, d_Q, st);
+  return launch_calq64_reduce(p, pl.nch, d_partial, d_Q, st, paired);
 }
 
 edb_status read_calq64x_status(int *status, bool clear) {

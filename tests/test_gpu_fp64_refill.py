@@ -45,3 +45,37 @@ def test_every_launch_shape_against_the_direct_sum(edb, oracle, N):
     finally:
         edb.set_wait_limit_ns(-1)
     assert np.array_equal(q.calQ(None, fin)[modes], got)
+
+
+@pytest.mark.parametrize("N", [8, 16, 17])
+def test_captured_and_back_to_back_sums_have_the_same_bits(edb, N):
+    """The three launches of a sum overlap; a graph of two sums in a chain, replayed
+    without waiting, and the same sums called one after another agree."""
+    import torch
+
+    rng = np.random.default_rng(N)
+    f = torch.from_numpy(rng.standard_normal(N ** 3) + 1j * rng.standard_normal(N ** 3)).cuda()
+    q = edb.QCalculator(N, 0, L=6.0, filter=False, index_mode=INDEX_ALIASED)
+    q.genB()
+    one, two = torch.empty_like(f), torch.empty_like(f)
+    q.calQ_device(f, one)
+    torch.cuda.synchronize()
+    q.calQ_device(one, two)
+    torch.cuda.synchronize()
+    a, b = torch.zeros_like(f), torch.zeros_like(f)
+    for _ in range(20):
+        q.calQ_device(f, a)
+        q.calQ_device(a, b)
+    torch.cuda.synchronize()
+    assert torch.equal(a, one) and torch.equal(b, two)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        st = torch.cuda.current_stream()
+        q.calQ_device(f, a, stream=st)
+        q.calQ_device(a, b, stream=st)
+    a.zero_()
+    b.zero_()
+    for _ in range(20):
+        g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(a, one) and torch.equal(b, two)
