@@ -451,7 +451,7 @@ def main():
             table = {0: nb, 1: nb, 2: (n2 + 1) * (n2 // 4 + 1) * 8 + Nf ** 3 * 16}[kind]
             # the kernel each kind runs on this ALIASED table (the double-float
             # one in the launch shape genB timed fastest)
-            kern = {0: "calq64p_kernel" if Nf % 4 == 0 else "calq64x_kernel",
+            kern = {0: "calq64p_kernel",
                     1: "calq64_kernel", 2: "calq64f_kernel"}[kind]
             res[name] = {"evals_per_s": 1.0 / t, "ms_per_eval": t * 1e3,
                          "B_stream_GBs": nb / t / 1e9,

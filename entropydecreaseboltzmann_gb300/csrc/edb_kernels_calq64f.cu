@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(THREADS, MINB)
   const int j2c = ok ? j2 : 0;
   const int j3_0 = r * RUN;
   const int chunk = blockIdx.z;
-  // visited l1 planes of the pair structure (see calq64x_kernel)
+  // visited l1 planes of the pair structure (see calq64p_kernel)
   const int k1f = (j1 - n + N) % N;
   const int plo = k1f / 2;
   const int nlist = plo + 1 + max(0, (k1f + N) / 2 - k1f);

@@ -248,7 +248,7 @@ edb_status edb_qcalc_set_fp64_kernel(edb_qcalc *q, int kind);
 
 /* Launch shape of the double-float kernel (EDB_FP64_EMULATED), no reference
  * counterpart: CTA size and register cap, for the output-pair form (the pair
- * table with N % 4 == 0) the table rows per ring slot, and the rule that sizes
+ * table) the table rows per ring slot, and the rule that sizes
  * the l-line chunks (the second half of the shapes repeats the first with
  * chunks from a model of the schedule).  genB times every shape on the table
  * and keeps the fastest.  shape >= 0 overrides that choice
