@@ -107,64 +107,58 @@ __global__ void __launch_bounds__(CALQ64_THREADS)
 // k_d - n - 1, flat index with stride N into the (2n+1)^3-filled array.
 // ALIASED mode: the centred index of FFTW index k is (k + n) mod N.
 // Bound by the latency of its loads and of its FP64 adds (up to 100 chunks of at
-// most 512 KB, out of L2).  Four lanes share an output, each summing a quarter of
-// the chunks in order with RED_AHEAD loads on their way; the quarters are added
-// in order.  With one thread per output and one load at a time the N = 16 sum
-// took 51.3 us, the N = 12 sum 35.4.
-constexpr int RED_PARTS = 4, RED_OUT = 32 / RED_PARTS, RED_WARPS = 4, RED_AHEAD = 8;
+// most 512 KB, out of L2).  A block has 32 outputs: its four warps load the next
+// 32 chunks, eight each, into shared memory while the first two add the last 32,
+// in order, the real and the imaginary parts.  Sum of N = 16 with one thread per
+// output and one load at a time 51.3 us, with four lanes per output that each
+// summed a quarter 43.2; against those lanes now N = 8 14.4 -> 12.5 us, 12 22.6 ->
+// 20.7, 24 257.7 -> 256.8, 32 1051 -> 1049 (and the bits of one sum in order).
+constexpr int RED_OUT = 32, RED_WARPS = 4, RED_AHEAD = 8, RED_ROUND = RED_WARPS * RED_AHEAD;
 __global__ void __launch_bounds__(32 * RED_WARPS)
     calq64_reduce_kernel(QParams p, int nchunk, const double2 *partial, double2 *Q) {
+  __shared__ double2 sh[RED_ROUND][RED_OUT];
   dep_wait();
   const int N = p.N, n = p.n;
-  const int lane = threadIdx.x & 31, part = lane / RED_OUT;
-  const long long k =
-      ((long long)blockIdx.x * RED_WARPS + (threadIdx.x >> 5)) * RED_OUT + lane % RED_OUT;
-  double sr = 0.0, si = 0.0;
-  if (k < p.NQ) {
-    int k1 = (int)(k / ((long long)N * N)), k2 = (int)((k / N) % N), k3 = (int)(k % N);
-    int q1, q2, q3;
-    if (p.mode == EDB_INDEX_REFERENCE) {
-      q1 = (k1 < n + 1) ? k1 + n : k1 - (n + 1);
-      q2 = (k2 < n + 1) ? k2 + n : k2 - (n + 1);
-      q3 = (k3 < n + 1) ? k3 + n : k3 - n - 1;
-    } else {
-      q1 = (k1 + n) % N;
-      q2 = (k2 + n) % N;
-      q3 = (k3 + n) % N;
-    }
-    const long long q = ((long long)q1 * N + q2) * N + q3;
-    if (q < p.KC) {
-      const int per = (nchunk + RED_PARTS - 1) / RED_PARTS;
-      const int c0 = min(nchunk, part * per), c1 = min(nchunk, c0 + per);
-      const double2 *src = partial + q;
-      for (int c = c0; c < c1; c += RED_AHEAD) {
-        double2 v[RED_AHEAD];
-#pragma unroll
-        for (int i = 0; i < RED_AHEAD; ++i)
-          v[i] = c + i < c1 ? src[(long long)(c + i) * p.KC] : make_double2(0.0, 0.0);
-#pragma unroll
-        for (int i = 0; i < RED_AHEAD; ++i) {
-          if (c + i < c1) {
-            sr += v[i].x;
-            si += v[i].y;
-          }
-        }
-      }
-    }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long k = (long long)blockIdx.x * RED_OUT + lane;
+  int k1 = (int)(k / ((long long)N * N)), k2 = (int)((k / N) % N), k3 = (int)(k % N);
+  int q1, q2, q3;
+  if (p.mode == EDB_INDEX_REFERENCE) {
+    q1 = (k1 < n + 1) ? k1 + n : k1 - (n + 1);
+    q2 = (k2 < n + 1) ? k2 + n : k2 - (n + 1);
+    q3 = (k3 < n + 1) ? k3 + n : k3 - n - 1;
+  } else {
+    q1 = (k1 + n) % N;
+    q2 = (k2 + n) % N;
+    q3 = (k3 + n) % N;
   }
-  double tr = sr, ti = si;
+  const long long q = ((long long)q1 * N + q2) * N + q3;
+  const bool in = k < p.NQ && q < p.KC;
+  const double2 *src = partial + q + (long long)warp * RED_AHEAD * p.KC;
+  double2 v[RED_AHEAD];
+  auto load = [&](int c) {  // chunks c + 8 warp .. + 7
 #pragma unroll
-  for (int j = 1; j < RED_PARTS; ++j) {
-    const double r = __shfl_sync(0xffffffffu, sr, lane % RED_OUT + j * RED_OUT);
-    const double i = __shfl_sync(0xffffffffu, si, lane % RED_OUT + j * RED_OUT);
-    tr += r;
-    ti += i;
+    for (int i = 0; i < RED_AHEAD; ++i)
+      if (in && c + warp * RED_AHEAD + i < nchunk) v[i] = src[(long long)(c + i) * p.KC];
+  };
+  double sum = 0.0;
+  load(0);
+  for (int c = 0; c < nchunk; c += RED_ROUND) {
+#pragma unroll
+    for (int i = 0; i < RED_AHEAD; ++i) sh[warp * RED_AHEAD + i][lane] = v[i];
+    __syncthreads();
+    load(c + RED_ROUND);
+    const int m = min(RED_ROUND, nchunk - c);
+    if (warp < 2) {
+      const double *x = reinterpret_cast<const double *>(&sh[0][lane]) + warp;
+#pragma unroll 8
+      for (int i = 0; i < m; ++i) sum += x[2 * RED_OUT * i];
+    }
+    __syncthreads();
   }
-  if (part == 0 && k < p.NQ) Q[k] = make_double2(tr, ti);
+  if (warp < 2 && k < p.NQ) reinterpret_cast<double *>(Q + k)[warp] = in ? sum : 0.0;
 }
-static unsigned red_blocks(long long NQ) {
-  return (unsigned)((NQ + RED_OUT * RED_WARPS - 1) / (RED_OUT * RED_WARPS));
-}
+static unsigned red_blocks(long long NQ) { return (unsigned)((NQ + RED_OUT - 1) / RED_OUT); }
 
 edb_status launch_calq64(const QParams &p, const double *d_B, const double2 *d_fin,
                          double2 *d_partial, double2 *d_Q, cudaStream_t st) {
