@@ -183,49 +183,37 @@ __device__ __forceinline__ void tc_st8(uint32_t a, const uint32_t (&w)[8]) {
                "r"(w[7])
                : "memory");
 }
-// Consecutive columns of this lane as packed pairs, asynchronously: tc_wait_ld
-// before any use.
-__device__ __forceinline__ void tc_ld8(uint32_t a, u64 *x) {
+// Consecutive columns of this lane, asynchronously: the outputs are the registers
+// that the load itself writes, and nothing reads them before tc_wait_ld.
+__device__ __forceinline__ void tc_ld8(uint32_t a, uint32_t *x) {
   asm volatile(
-      "{\n .reg .b32 r<8>;\n"
-      " tcgen05.ld.sync.aligned.32x32b.x8.b32 {r0, r1, r2, r3, r4, r5, r6, r7}, [%4];\n"
-      " mov.b64 %0, {r0, r1};\n"
-      " mov.b64 %1, {r2, r3};\n"
-      " mov.b64 %2, {r4, r5};\n"
-      " mov.b64 %3, {r6, r7};\n"
-      "}\n"
-      : "=l"(x[0]), "=l"(x[1]), "=l"(x[2]), "=l"(x[3])
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3]), "=r"(x[4]), "=r"(x[5]), "=r"(x[6]),
+        "=r"(x[7])
       : "r"(a));
 }
-__device__ __forceinline__ void tc_ld16(uint32_t a, u64 *x) {
+__device__ __forceinline__ void tc_ld16(uint32_t a, uint32_t *x) {
   asm volatile(
-      "{\n .reg .b32 r<16>;\n"
-      " tcgen05.ld.sync.aligned.32x32b.x16.b32 {r0, r1, r2, r3, r4, r5, r6, r7, r8, r9, r10, r11, r12, r13, r14, r15}, [%8];\n"
-      " mov.b64 %0, {r0, r1};\n"
-      " mov.b64 %1, {r2, r3};\n"
-      " mov.b64 %2, {r4, r5};\n"
-      " mov.b64 %3, {r6, r7};\n"
-      " mov.b64 %4, {r8, r9};\n"
-      " mov.b64 %5, {r10, r11};\n"
-      " mov.b64 %6, {r12, r13};\n"
-      " mov.b64 %7, {r14, r15};\n"
-      "}\n"
-      : "=l"(x[0]), "=l"(x[1]), "=l"(x[2]), "=l"(x[3]), "=l"(x[4]), "=l"(x[5]), "=l"(x[6]), "=l"(x[7])
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, "
+      "%12, %13, %14, %15}, [%16];"
+      : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3]), "=r"(x[4]), "=r"(x[5]), "=r"(x[6]),
+        "=r"(x[7]), "=r"(x[8]), "=r"(x[9]), "=r"(x[10]), "=r"(x[11]), "=r"(x[12]), "=r"(x[13]),
+        "=r"(x[14]), "=r"(x[15])
       : "r"(a));
 }
 template <int CH>
-__device__ __forceinline__ void tc_ld(uint32_t a, u64 *x) {
+__device__ __forceinline__ void tc_ld(uint32_t a, uint32_t *x) {
   tc_ld16(a, x);
-  if constexpr (CH == 24) tc_ld8(a + 16, x + 8);
-  if constexpr (CH == 32) tc_ld16(a + 16, x + 8);
+  if constexpr (CH == 24) tc_ld8(a + 16, x + 16);
+  if constexpr (CH == 32) tc_ld16(a + 16, x + 16);
 }
 // Completes this thread's loads; the registers pass through so that no use of
-// them is scheduled before it.
-template <int H>
-__device__ __forceinline__ void tc_wait_ld(u64 (&x)[H]) {
+// them (packing them into pairs among those) is scheduled before it.
+template <int CH>
+__device__ __forceinline__ void tc_wait_ld(uint32_t (&x)[CH]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-  for (int j = 0; j < H; ++j) asm volatile("" : "+l"(x[j]));
+  for (int j = 0; j < CH; ++j) asm volatile("" : "+r"(x[j]));
 }
 
 // One lane of the (converged) warp.
@@ -259,6 +247,11 @@ __device__ __forceinline__ void two_sum(float &hi, float &lo, float x) {
 __device__ __forceinline__ float2 upk(u64 v) {
   float2 r;
   asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ u64 pk(uint32_t a, uint32_t b) {
+  u64 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(a), "r"(b));
   return r;
 }
 __device__ __forceinline__ void fma2(u64 &acc, u64 a, u64 b) {
@@ -335,8 +328,9 @@ struct TcCfg {
   static constexpr int NU0 = (512 - AC) / UC;
   static constexpr int NU = NU0 > 6 ? 6 : NU0;    // tile units
   static constexpr int CH = NC == 32 ? 16 : NC == 24 ? 24 : 32;  // columns per read of a tile
-  // registers of a compute and of a service thread (2 RC + 2 RS = 4 x 128)
-  static constexpr int RC = 192, RS = 256 - RC;
+  // registers of a compute and of a service thread (2 RC + 2 RS = 4 x 128); at 192
+  // the largest form spills 76 bytes, at 200 the others' service threads do
+  static constexpr int RC = NC == 32 && SG == 4 ? 200 : 192, RS = 256 - RC;
   static constexpr int NPB = NC == 32 ? 1 : 2;    // staged f_L planes
   static constexpr int SB = 128 * NC * 4;         // bytes of a step's weights
   static constexpr int PITCH = NC + 1;            // floats per lane of the fold's staging
@@ -452,7 +446,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) calqtc_kernel(const TcArgs a) {
     for (int e = tid; e < SG * NN; e += 256) sums[e] = make_float4(0.f, 0.f, 0.f, 0.f);
     asm volatile("bar.sync 1, 256;" ::: "memory");
     u64 acc[SW][NC], b[NC / 2];  // re then im pairs; weights
-    u64 x[2][CH / 2];
+    uint32_t x[2][CH];
 #pragma unroll
     for (int s = 0; s < SW; ++s)
 #pragma unroll
@@ -465,7 +459,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) calqtc_kernel(const TcArgs a) {
                      : "r"(myB + (uint32_t)(stg * Cfg::SB + j * 2048)));
     };
     // read k of this warpgroup's tile i of unit u
-    auto read = [&](int u, int i, int k, u64 (&d)[CH / 2]) {
+    auto read = [&](int u, int i, int k, uint32_t (&d)[CH]) {
       tc_ld<CH>(d0 + (uint32_t)(u * Cfg::UC + 2 * i * Cfg::DC + k * CH), d);
     };
     constexpr bool even = (SW * K) % 2 == 0;
@@ -474,7 +468,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) calqtc_kernel(const TcArgs a) {
     // first read of the next unit (after the last step: of a unit that does not
     // come, without waiting; every read and load is unconditional so that no
     // register is kept for the path without it)
-    auto first = [&](u64 (&d)[CH / 2], bool last) {
+    auto first = [&](uint32_t (&d)[CH], bool last) {
       mbar_wait(bar(DF + du), dp, lim, rd | last);
       tc_fence_after();
       read(du, 0, 0, d);
@@ -500,7 +494,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) calqtc_kernel(const TcArgs a) {
       for (int s = 0; s < SW; ++s) {
 #pragma unroll
         for (int k = 0; k < K; ++k) {
-          u64 (&cur)[CH / 2] = x[(s * K + k) & 1], (&nxt)[CH / 2] = x[(s * K + k + 1) & 1];
+          uint32_t (&cur)[CH] = x[(s * K + k) & 1], (&nxt)[CH] = x[(s * K + k + 1) & 1];
           // the next read is on its way while this one is used
           tc_wait_ld(cur);
           if (k + 1 < K) {
@@ -523,7 +517,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) calqtc_kernel(const TcArgs a) {
 #pragma unroll
           for (int j = 0; j < CH / 2; ++j) {
             const int c = k * (CH / 2) + j;
-            fma2(acc[s][c], b[c % (NC / 2)], cur[j]);
+            fma2(acc[s][c], b[c % (NC / 2)], pk(cur[2 * j], cur[2 * j + 1]));
           }
         }
         // the step's weights are in registers: lane 0 saw them land

@@ -1,0 +1,31 @@
+"""Reads of asynchronous results in the tensor-core batched kernel's source.
+
+What a tensor-memory load writes may not be touched before the wait that
+completes it.  Code that breaks this can give right answers for as long as the
+assembler happens to order it, so the source itself is checked.
+"""
+import os
+import re
+
+import entropydecreaseboltzmann_gb300
+
+SOURCE = os.path.join(os.path.dirname(entropydecreaseboltzmann_gb300.__file__), "csrc",
+                      "edb_kernels_calqtc.cu")
+
+
+def _text():
+    with open(SOURCE) as f:
+        return f.read()
+
+
+def _asm(text):
+    """The instruction text of every asm statement."""
+    blocks = re.findall(r"asm(?: volatile)?\(\s*((?:\"(?:[^\"\\\\]|\\\\.)*\"\s*)+)", text)
+    return ["".join(re.findall(r"\"((?:[^\"\\\\]|\\\\.)*)\"", b)) for b in blocks]
+
+
+def test_a_tensor_memory_load_stands_alone_in_its_asm_statement():
+    loads = [a for a in _asm(_text()) if "tcgen05.ld" in a]
+    assert len(loads) == 2
+    for a in loads:
+        assert a.count(";") == 1 and "mov" not in a, a
