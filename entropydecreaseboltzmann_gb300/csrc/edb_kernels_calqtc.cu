@@ -531,8 +531,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1) calqtc_kernel(const TcArgs a) {
       load_b(st);
       if (--fc == 0 || i + 1 == total) {
         // fold: the lanes of an output are added, then joined to its
-        // compensated (hi, lo) sum
+        // compensated (hi, lo) sum.  The read ahead is completed first: after
+        // the last step nothing else does, and its registers are free for the
+        // code below.
         fc = a.FL;
+        tc_wait_ld(x[0]);
 #pragma unroll
         for (int s = 0; s < SW; ++s) {
           float *own = reinterpret_cast<float *>(sums + ((s / TW) * TP + (s % TW) * 2 + h) * NN);

@@ -29,3 +29,12 @@ def test_a_tensor_memory_load_stands_alone_in_its_asm_statement():
     assert len(loads) == 2
     for a in loads:
         assert a.count(";") == 1 and "mov" not in a, a
+
+
+def test_the_read_ahead_of_the_last_step_is_completed():
+    # the read ahead always fills x[0]: nothing of the fold, which ends the
+    # last step, comes before its wait
+    fold = _text().split("if (--fc == 0 || i + 1 == total) {")
+    assert len(fold) == 2
+    code = re.sub(r"//[^\n]*", "", fold[1])
+    assert re.match(r"\s*fc = a\.FL;\s*tc_wait_ld\(x\[0\]\);", code)
