@@ -520,8 +520,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1) calqtc_kernel(const TcArgs a) {
             fma2(acc[s][c], b[c % (NC / 2)], pk(cur[2 * j], cur[2 * j + 1]));
           }
         }
-        // the step's weights are in registers: lane 0 saw them land
-        if (s == 0) mbar_arrive(bar(BE + stc), lane == 0 && lim != 0);
+        // the step's weights are in the registers of every lane, and lane 0 saw
+        // them land
+        if (s == 0) {
+          __syncwarp();
+          mbar_arrive(bar(BE + stc), lane == 0 && lim != 0);
+        }
       }
       if (!even) {
         first(x[0], last);
@@ -621,6 +625,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) calqtc_kernel(const TcArgs a) {
         }
         l2 = l2 == 0 ? N - 1 : l2 - 1;
       }
+      __syncwarp();
       mbar_arrive(bar(PE + pb), lane == 0);
       if (++pb == NPB) {
         pb = 0;

@@ -38,3 +38,11 @@ def test_the_read_ahead_of_the_last_step_is_completed():
     assert len(fold) == 2
     code = re.sub(r"//[^\n]*", "", fold[1])
     assert re.match(r"\s*fc = a\.FL;\s*tc_wait_ld\(x\[0\]\);", code)
+
+
+def test_one_lane_gives_shared_memory_back_only_after_the_whole_warp():
+    # BE: a stage of weights, PE: a staged plane; both are read by all lanes
+    releases = re.findall(r"([^\n]*)\n\s*mbar_arrive\(bar\((?:BE|PE) ", _text())
+    assert len(releases) == 2
+    for line in releases:
+        assert line.strip() == "__syncwarp();", line
