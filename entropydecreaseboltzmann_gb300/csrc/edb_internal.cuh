@@ -269,6 +269,9 @@ edb_status read_calq64x_status(int *status, bool clear);
 // Limit of every bounded mbarrier wait of the Q-hat kernels, passed to each
 // launch (default 200 ms; see edb_set_wait_limit_ns).
 unsigned long long wait_limit_ns();
+// Limit of the drain after a wait ran out: the block then waits this long at
+// most for each copy and matrix product it issued, so none lands after it exits.
+constexpr unsigned long long DRAIN_LIMIT_NS = 1000000000ull;
 
 // Batched cubic DFT (FP64 or FP32), out-of-place; d_tmp holds batch*N^3 complex.
 edb_status launch_dft3d(int N, int batch, const void *d_in, void *d_out, void *d_tmp,

@@ -240,9 +240,6 @@ constexpr int ROWPAD = 8;                 // floats after each B-tile row
 constexpr int FLPAD = 2;                  // complex after each f_l line
 constexpr int PLPAD = 2;                  // complex after each solve's plane
 constexpr int FOLD_LINES = 4;             // l-lines per compensated fold
-// Limit of the drain after a wait ran out: the block then waits this long at
-// most for each copy it issued, so none lands after it exits.
-constexpr unsigned long long DRAIN_LIMIT_NS = 1000000000ull;
 
 __device__ int g_calq32_status;  // nonzero: a bounded wait ran out
 

@@ -65,9 +65,6 @@ using namespace df;
 constexpr int RUN = 4;  // outputs per thread along j3
 
 constexpr int DEPTH = 8;  // B rows in flight per warp
-// Limit of the drain after a wait ran out: lane 0 then waits this long at
-// most for each copy its warp issued, so none lands after the block exits.
-constexpr unsigned long long DRAIN_LIMIT_NS = 1000000000ull;
 
 __device__ __forceinline__ uint32_t s_addr(const void *p) {
   return (uint32_t)__cvta_generic_to_shared(p);

@@ -53,7 +53,6 @@ typedef unsigned long long u64;
 constexpr int TC_THREADS = 512;
 constexpr int TC_HDR = 1024;
 constexpr int MAX_STG = 8;
-constexpr unsigned long long TC_DRAIN_NS = 20000000ull;
 
 __device__ __forceinline__ uint32_t s_addr(const void *p) {
   return (uint32_t)__cvta_generic_to_shared(p);
@@ -682,9 +681,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) calqtc_kernel(const TcArgs a) {
         ob ^= 1;
         op ^= (ob == 0);
       }
-      // every MMA and every commit has landed before the block leaves
+      // every MMA and every commit has landed before the block leaves; one that
+      // has not is reported as a wait that ran out
       tc_commit(bar(XD), el);
-      mbar_poll(bar(XD), 0, TC_DRAIN_NS);
+      if (!mbar_poll(bar(XD), 0, DRAIN_LIMIT_NS)) lim = 0;
     } else if (warp == 13) {
       // ------------------------------------------------------ weight stream
       const char *src = reinterpret_cast<const char *>(a.B32) +
@@ -809,7 +809,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) calqtc_kernel(const TcArgs a) {
       // the last copy issued into each stage may still be landing
       const int n = *issued;
       for (int i = max(0, n - a.NST); i < n; ++i)
-        mbar_poll(bar(BF + i % a.NST), (uint32_t)((i / a.NST) & 1), TC_DRAIN_NS);
+        mbar_poll(bar(BF + i % a.NST), (uint32_t)((i / a.NST) & 1), DRAIN_LIMIT_NS);
     }
   } else {
     const float4 *sums = reinterpret_cast<const float4 *>(smem + o_sum);

@@ -46,3 +46,14 @@ def test_one_lane_gives_shared_memory_back_only_after_the_whole_warp():
     assert len(releases) == 2
     for line in releases:
         assert line.strip() == "__syncwarp();", line
+
+
+def test_the_drain_after_a_wait_ran_out_has_one_limit_and_its_outcome_counts():
+    csrc = os.path.dirname(SOURCE)
+    limits = []
+    for name in sorted(os.listdir(csrc)):
+        with open(os.path.join(csrc, name)) as f:
+            limits += re.findall(r"constexpr unsigned long long (\w*DRAIN\w*) = (\d+)ull;", f.read())
+    assert limits == [("DRAIN_LIMIT_NS", "1000000000")]
+    # matrix products still in flight: the launch reports it
+    assert "if (!mbar_poll(bar(XD), 0, DRAIN_LIMIT_NS)) lim = 0;" in _text()
