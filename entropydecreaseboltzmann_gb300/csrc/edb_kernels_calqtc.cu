@@ -34,9 +34,14 @@
 // stage the next f_L plane.  Every hand-over is an mbarrier and every wait is
 // bounded.
 //
-// Summation: plain FP32 over blocks of 4 N terms, then the lanes of an output
-// are added and the block joins a compensated (hi, lo) sum: the blocks and the
-// compensation of calq32_kernel.
+// Summation: plain FP32 over 5 N / 2 terms in a lane, then over the CL lanes of
+// an output; the result joins a compensated (hi, lo) sum.  No term takes part in
+// as many plain additions as in calq32_kernel (4 N), and the error against 64
+// bits is below that kernel's at every size.  Relative L2, that kernel -> this
+// one (with 4 N terms in a lane): white noise, N = 13 1.63e-7 -> 1.54e-7 (1.83e-7),
+// 17 1.87e-7 -> 1.64e-7 (1.94e-7), 31 2.46e-7 -> 1.91e-7 (2.35e-7); BKW with a bump,
+// N = 13 5.9e-7 -> 5.1e-7 (6.6e-7), 21 8.5e-7 -> 7.0e-7 (8.3e-7).  The shorter sums
+// cost 1.5 to 6% (4096 of N = 13 9.20 -> 9.54 ms, 37 of N = 21 770 -> 806 us).
 //
 // What bounds it: the instruction issue of the hand-overs and of the A rows
 // beside the FMAs (a tile of N = 24 takes about 240 clocks an SM, its FMAs 60).
@@ -44,6 +49,7 @@
 // 0.80, 256 of N = 31 126 -> 31, 16 of N = 17 0.82 -> 0.16.
 #include <algorithm>
 
+#include "edb_df.cuh"
 #include "edb_internal.cuh"
 
 namespace edb {
@@ -553,26 +559,30 @@ __global__ void __launch_bounds__(TC_THREADS, 1) calqtc_kernel(const TcArgs a) {
               acc[s][c2 * (NC / 2) + j] = 0ull;
             }
             asm volatile("bar.sync %0, 128;" ::"r"(2 + h) : "memory");
-            // warp q: outputs k2 = q, q + 4, ..., three at a time; lane k3
+            // warp q: outputs k2 = q, q + 4, ..., UR at a time; lane k3
             if (lane < N) {
-              for (int k0 = q; k0 < N; k0 += 12) {
-                float y[3] = {0.f, 0.f, 0.f};
-                const float *y0[3];
+              constexpr int UR = NC == 24 ? 6 : 4;  // a warp has up to NC / 4 of them
+              for (int k0 = q; k0 < N; k0 += 4 * UR) {
+                u64 y[UR / 2] = {};  // of two outputs each
+                const float *y0[UR];
 #pragma unroll
-                for (int u = 0; u < 3; ++u) y0[u] = stage + min(k0 + 4 * u, N - 1) * CL * P1;
+                for (int u = 0; u < UR; ++u) y0[u] = stage + min(k0 + 4 * u, N - 1) * CL * P1;
                 int j = lane;
                 for (int c = 0; c < CL; ++c) {
 #pragma unroll
-                  for (int u = 0; u < 3; ++u) y[u] += y0[u][c * P1 + j];
+                  for (int u = 0; u < UR / 2; ++u)
+                    y[u] = df::add2(y[u], pk(__float_as_uint(y0[2 * u][c * P1 + j]),
+                                             __float_as_uint(y0[2 * u + 1][c * P1 + j])));
                   j = j == 0 ? N - 1 : j - 1;
                 }
 #pragma unroll
-                for (int u = 0; u < 3; ++u) {
+                for (int u = 0; u < UR; ++u) {
                   const int k2 = k0 + 4 * u;
                   if (k2 < N) {
                     float2 *hl = reinterpret_cast<float2 *>(own + 4 * (k2 * N + lane) + 2 * c2);
+                    const float2 yy = upk(y[u / 2]);
                     float2 t = *hl;
-                    two_sum(t.x, t.y, y[u]);
+                    two_sum(t.x, t.y, u & 1 ? yy.y : yy.x);
                     *hl = t;
                   }
                 }
@@ -864,7 +874,7 @@ edb_status launch_calqtc(int N, int S, const float *d_B32, const float2 *d_fin, 
   a.V = g.V;
   a.pitch = g.pitch;
   a.C = C;
-  a.FL = 4 * N;
+  a.FL = 5 * N / 2;
   a.B32 = d_B32;
   a.fin = d_fin;
   a.Q = d_Q;
