@@ -471,10 +471,14 @@ __global__ void __launch_bounds__(MAXT, MINB)
 // N = 9 26.9 -> 22.7 us, 17 84 -> 70, 18 105 -> 85, 23 312 -> 260, 25 503 -> 417,
 // 27 757 -> 563, 31 1386 -> 1156.  That form kept the products with f_l.re and
 // f_l.im apart; one accumulator for both makes the low parts twice as long a
-// sum, so they are folded back every other step (3% of the time).  Relative
-// error against the FP64 kernel on near-equilibrium data, that form -> folded
-// (unfolded): N = 9 1.7e-14 -> 2.2e-14 (3.0e-14), 17 5.0e-14 -> 2.6e-14 (8.6e-14),
-// 23 9.1e-14 -> 3.6e-14 (1.6e-13), 30 6.7e-13 -> 6.8e-14 (6.5e-13).
+// sum, so they are folded back every other step (3% of the time), and after
+// each product below N = 14 (RAG 2), where a sum is too short for the former to
+// make up for it (N = 9 13.1 -> 13.2 us of device time, 13 22.5 -> 23.3).  Relative
+// error against the FP64 kernel, mean of 400 solves, (re, im) form -> now (folded
+// every other step): BKW with a bump N = 6 8.5e-15 -> 7.8e-15 (9.1e-15), 9 6.5e-14 ->
+// 6.0e-14 (7.0e-14), 13 2.7e-14 -> 2.3e-14 (2.7e-14), 15 3.8e-14 -> 3.2e-14, 17 9.8e-14
+// -> 5.4e-14; white noise N = 5 4.4e-15 -> 4.3e-15 (4.9e-15), 10 5.9e-15 -> 5.1e-15
+// (6.1e-15); unfolded it grew to 1.6e-13 at N = 23 and is 3.6e-14 now.
 // Launches: the kernel starts as the split of f-hat ends (its own start and the
 // first table rows run under that kernel's end), and the reduction as this one
 // ends: N = 8 20.6 -> 14.4 us a sum, 12 27.8 -> 22.6, 16 40.4 -> 35.1, 17 69.7 ->
@@ -496,7 +500,7 @@ __host__ __device__ constexpr int p64_box_threads(int threads) {
 // tmB: the table as N^3 rows of 2 N^3 floats, box ROWS rows of a full warp's
 // segment (the last warp, where it is short, copies a full box too: the columns
 // past its own are other threads' and are not read).
-template <int MAXT, int MINB, int ROWS, int NC, bool RAG>
+template <int MAXT, int MINB, int ROWS, int NC, int RAG>
 __global__ void __launch_bounds__(MAXT, MINB)
     calq64p_kernel(QParams p, int J2T, int LC, const float4 *fdr, double2 *partial,
                    unsigned long long wait_ns, const __grid_constant__ CUtensorMap tmB) {
@@ -690,11 +694,15 @@ __global__ void __launch_bounds__(MAXT, MINB)
           const u64 nuim = mul2(nbh, eh[s][1]);
           const u64 ucim = fma2(bh, el[s][1], fma2(bl, eh[s][1], fma2(bh, eh[s][1], nuim)));
           df_axpy(accR[h], xr, nxr, nlr, nure, ucre);  // + f_l.re u.re
-          df_axpy(accR[h], nxi, xi, li, nuim, ucim);   // - f_l.im u.im
           df_axpy(accI[h], xr, nxr, nlr, nuim, ucim);  // + f_l.re u.im
+          if constexpr (RAG == 2) {
+            df_renorm(accR[h]);
+            df_renorm(accI[h]);
+          }
+          df_axpy(accR[h], nxi, xi, li, nuim, ucim);   // - f_l.im u.im
           df_axpy(accI[h], xi, nxi, nli, nure, ucre);  // + f_l.im u.re
         }
-        if (RAG && t % 2 == 1) {  // see above
+        if (RAG == 2 || (RAG == 1 && t % 2 == 1)) {  // see above
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             df_renorm(accR[h]);
@@ -771,12 +779,12 @@ typedef void (*C64pFn)(QParams, int, int, const float4 *, double2 *, unsigned lo
 template <int S>
 static C64pFn c64p_fn_s(int N) {
   constexpr int T = kC64pShapes[S].maxt, B = kC64pShapes[S].minb, R = kC64pShapes[S].rows;
-  if (N % RUN) return calq64p_kernel<T, B, R, 0, true>;
-  if (N == 20) return calq64p_kernel<T, B, R, 20, false>;
-  if (N == 24) return calq64p_kernel<T, B, R, 24, false>;
-  if (N == 28) return calq64p_kernel<T, B, R, 28, false>;
-  if (N == 32) return calq64p_kernel<T, B, R, 32, false>;
-  return calq64p_kernel<T, B, R, 0, false>;
+  if (N % RUN) return N < 14 ? calq64p_kernel<T, B, R, 0, 2> : calq64p_kernel<T, B, R, 0, 1>;
+  if (N == 20) return calq64p_kernel<T, B, R, 20, 0>;
+  if (N == 24) return calq64p_kernel<T, B, R, 24, 0>;
+  if (N == 28) return calq64p_kernel<T, B, R, 28, 0>;
+  if (N == 32) return calq64p_kernel<T, B, R, 32, 0>;
+  return calq64p_kernel<T, B, R, 0, 0>;
 }
 static C64pFn c64p_fn(int shape, int N) {
   switch (shape) {
