@@ -214,6 +214,8 @@ struct TcGeom {
   int CL, V, NC, pitch;
 };
 TcGeom tc_geom(int N);
+// Of S solves in C chunks on sms SMs, those that go in CTAs of four solves.
+int tc_fours(int S, int N, int C, int sms);
 inline long long c32_table_floats(int N) {
   if (tc_takes(N)) {
     const TcGeom g = tc_geom(N);

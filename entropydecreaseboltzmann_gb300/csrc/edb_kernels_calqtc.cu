@@ -864,6 +864,36 @@ static edb_status launch_tc(const TcArgs &args, int first, int end, cudaStream_t
   return EDB_OK;
 }
 
+// Solves per CTA: 4 for the first tc_fours() solves and 2 for the others, in a
+// launch of their own, by the number of CTA waves.  A wave of CTAs of 2 takes
+// 0.67 of one of 4 at 16 weight columns and 0.63 above (N = 13 74 | 109 us, 21
+// 311 | 492, 31 1476 | 2285): 37 x N = 21 944 us in CTAs of 4 (210 of them on 152
+// SMs), 887 in CTAs of 2, 795 as 28 + 9; 17 x N = 31 4.44 -> 2.86 ms, 30 x N = 25
+// 1.90 -> 1.59 ms.  A second launch has to gain 3% and its start: over many waves
+// the CTAs drift apart, and a last one that is part full costs less (500 x N = 21
+// 8.45 ms, 8.55 as 492 + 8).
+// Each wave of fours given up costs at least 0.26 of a wave and all of them
+// together gain less than the last part-full one, so only the last few waves'
+// groups are tried: 4096 x N = 13 11.5 -> 8 us of host time a call, 40,000 58 -> 9.
+int tc_fours(int S, int N, int C, int sms) {
+  const double two = tc_geom(N).NC == 16 ? 0.67 : 0.63;
+  const long long per = (long long)N * C;
+  auto waves = [&](long long groups) { return (double)((groups * per + sms - 1) / sms); };
+  const int all = (S + 3) / 4, wave = (int)(sms / per) + 1;  // groups, at least a wave's
+  int four = S;
+  double best = 1e30;
+  for (int g4 = all; g4 >= std::max(0, all - 8 * wave); --g4) {
+    const int n4 = std::min(S, 4 * g4), n2 = S - n4;
+    double t = waves(g4) + two * waves((n2 + 1) / 2);
+    if (n2 > 0 && n4 > 0) t = 1.03 * t + 0.02;
+    if (t < best - 1e-9) {
+      best = t;
+      four = n4;
+    }
+  }
+  return four;
+}
+
 edb_status launch_calqtc(int N, int S, const float *d_B32, const float2 *d_fin, float2 *d_Q, int C,
                          float4 *d_partial, cudaStream_t st) {
   const TcGeom g = tc_geom(N);
@@ -882,28 +912,7 @@ edb_status launch_calqtc(int N, int S, const float *d_B32, const float2 *d_fin, 
   a.wait_ns = wait_limit_ns();
   EDB_TRY(calq32_status_ptr(&a.status));
   a.NST = 0;
-  // Solves per CTA: 4 for the first `four` solves and 2 for the others, in a
-  // launch of their own, by the number of CTA waves.  A wave of CTAs of 2 takes
-  // 0.67 of one of 4 at 16 weight columns and 0.63 above (N = 13 74 | 109 us, 21
-  // 311 | 492, 31 1476 | 2285): 37 x N = 21 944 us in CTAs of 4 (210 of them on 152
-  // SMs), 887 in CTAs of 2, 795 as 28 + 9; 17 x N = 31 4.44 -> 2.86 ms, 30 x N = 25
-  // 1.90 -> 1.59 ms.  A second launch has to gain 3% and its start: over many waves
-  // the CTAs drift apart, and a last one that is part full costs less (500 x N = 21
-  // 8.45 ms, 8.55 as 492 + 8).
-  const long long per = (long long)N * C, sms = device_sm_count();
-  auto waves = [&](long long groups) { return (double)((groups * per + sms - 1) / sms); };
-  const int all = (S + 3) / 4;
-  int four = S;
-  double best = 1e30;
-  for (int g4 = all; g4 >= 0; --g4) {
-    const int n4 = std::min(S, 4 * g4), n2 = S - n4;
-    double t = waves(g4) + (g.NC == 16 ? 0.67 : 0.63) * waves((n2 + 1) / 2);
-    if (n2 > 0 && n4 > 0) t = 1.03 * t + 0.02;
-    if (t < best - 1e-9) {
-      best = t;
-      four = n4;
-    }
-  }
+  const int four = tc_fours(S, N, C, device_sm_count());
 #define EDB_TC(NC)                                \
   EDB_TRY((launch_tc<NC, 4>(a, 0, four, st)));    \
   return launch_tc<NC, 2>(a, four, S, st)
