@@ -134,6 +134,8 @@ struct edb_qcalc {
   size_t pairs_bytes = 0;
 };
 
+static std::atomic<int> g_qcalcs{0};  // live handles
+
 // Grows the qcalc's solve-pair buffer to hold S solves (not under capture).
 static edb_status qcalc_pairs(edb_qcalc *q, int S) {
   if (tc_takes(q->d.N)) return EDB_OK;  // no pair layout there
@@ -196,6 +198,7 @@ extern "C" edb_status edb_qcalc_create(const edb_qcalc_desc *d, edb_qcalc **out)
     delete q;
     return cuda_fail(e, "cudaStreamCreate");
   }
+  ++g_qcalcs;
   *out = q;
   return EDB_OK;
 }
@@ -215,6 +218,7 @@ extern "C" edb_status edb_qcalc_destroy(edb_qcalc *q) {
   dfree(q->Q);
   if (q->st) cudaStreamDestroy(q->st);
   delete q;
+  if (--g_qcalcs == 0) calq32_queue_trim();
   return EDB_OK;
 }
 

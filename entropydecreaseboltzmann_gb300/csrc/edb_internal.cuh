@@ -227,6 +227,8 @@ inline long long c32_table_floats(int N) {
 // Results in Q (C == 1) or, per chunk, in partial (calq32_reduce_kernel's form).
 edb_status launch_calqtc(int N, int S, const float *d_B32, const float2 *d_fin, float2 *d_Q, int C,
                          float4 *d_partial, cudaStream_t st);
+// Gives back what the batched launches' queue counters have left in their pool.
+void calq32_queue_trim();
 // The batched kernels' status word on the current device.
 edb_status calq32_status_ptr(int **p);
 // variant in [0, calq32_variants()) selects the solve group and CTA shape

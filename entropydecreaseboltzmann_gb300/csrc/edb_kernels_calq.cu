@@ -1690,17 +1690,22 @@ edb_status launch_calq32_batch(int N, int S, const float *d_B32, const float2 *d
 // comes from a pool of the library's own that keeps up to 64 MB across
 // synchronisations; the default pool gives its memory back at each one, and a
 // caller that waits for every call then paid for a device allocation each
-// time (180 us a call).  Under capture it is an allocation node.
+// time (180 us a call).  The pool gives its memory back when the last handle goes
+// (calq32_queue_trim).  Under capture the counter is an allocation node.
+static std::mutex g_queue_mu;
+static std::map<int, cudaMemPool_t> &queue_pools() {  // by device; never destroyed
+  static auto *pools = new std::map<int, cudaMemPool_t>;
+  return *pools;
+}
 static edb_status queue_alloc(unsigned long long **p, cudaStream_t st) {
-  static std::mutex mu;
-  static std::map<int, cudaMemPool_t> pools;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   EDB_CUDA(cudaStreamIsCapturing(st, &cap));
   cudaMemPool_t pool = nullptr;
   if (cap == cudaStreamCaptureStatusNone) {
     int dev = 0;
     EDB_CUDA(cudaGetDevice(&dev));
-    std::lock_guard<std::mutex> lock(mu);
+    std::lock_guard<std::mutex> lock(g_queue_mu);
+    auto &pools = queue_pools();
     auto it = pools.find(dev);
     if (it == pools.end()) {
       cudaMemPoolProps pr = {};
@@ -1721,6 +1726,10 @@ static edb_status queue_alloc(unsigned long long **p, cudaStream_t st) {
     EDB_CUDA(cudaMallocAsync(reinterpret_cast<void **>(p), sizeof(**p), st));
   EDB_CUDA(cudaMemsetAsync(*p, 0, sizeof(**p), st));
   return EDB_OK;
+}
+void calq32_queue_trim() {
+  std::lock_guard<std::mutex> lock(g_queue_mu);
+  for (const auto &d : queue_pools()) cudaMemPoolTrimTo(d.second, 0);
 }
 
 template <int V>
