@@ -250,7 +250,7 @@ static edb_status qcalc_split_B2(edb_qcalc *q) {
 static edb_status qcalc_alloc_work(edb_qcalc *q) {
   if (!q->partial) {
     q->nchunk = calq64_nchunk(q->p);
-    int nmax = calq64x_nchunk(q->p, nullptr);
+    int nmax = calq64x_nchunk(q->p, qcalc_b2_paired(q));
     if (q->nchunk > nmax) nmax = q->nchunk;
     if (qcalc_b2_paired(q)) nmax = std::max(nmax, calq64f_nchunk(q->p));
     EDB_TRY(dalloc(&q->partial, (size_t)nmax * q->p.KC));

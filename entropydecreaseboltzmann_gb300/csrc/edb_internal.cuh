@@ -158,8 +158,8 @@ __device__ __forceinline__ void dep_launch() {
 // FP64-accurate calQ on the FP32 pipe (double-float arithmetic): B2 is the
 // table split into (hi, lo) floats, fdf (N^3 float4) the input split into
 // {re_hi, im_hi, re_lo, im_lo}.
-// d_partial holds calq64x_nchunk(p) * KC.
-int calq64x_nchunk(const QParams &p, int *J2T_out);
+// d_partial holds calq64x_nchunk(p, paired) * KC.
+int calq64x_nchunk(const QParams &p, bool paired);
 // FP32 tiled tensor map, no swizzle, out-of-bounds elements read as zero;
 // false: the driver has no encoder or refused the map.
 bool encode_map(CUtensorMap *m, int rank, const void *base, const cuuint64_t *dim,

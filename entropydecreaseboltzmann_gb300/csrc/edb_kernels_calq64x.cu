@@ -39,13 +39,12 @@
 // c64x_plan_compute).  Each CTA writes
 // FP64 partial sums per chunk; calq64_reduce_kernel adds the chunks in order.
 //
-// B stream: when every warp's row segment is a contiguous, 16-byte aligned run
-// (calq64p_kernel always; here P % 4 == 0 and whole j2 tiles), each warp streams
-// its own 1 KB segment of the next D rows into a private shared-memory ring with
-// TMA copies (boxes of rows there, 1-D bulk copies here; lane 0 issues; one
+// B stream: calq64p_kernel's warps each stream their own 1 KB segment of the next
+// rows into a private shared-memory ring with tensor copies (lane 0 issues; one
 // mbarrier per slot; waits bounded by %globaltimer, a timeout sets the device
-// status word).  Otherwise threads load their 32 bytes per row with __ldg, one
-// row ahead.
+// status word).  calq64x_kernel's rows have an odd length (P = N - 1), so that
+// no segment is aligned: its threads load their 32 bytes per row with __ldg,
+// one row ahead.
 #include <cuda.h>
 
 #include <algorithm>
@@ -64,27 +63,12 @@ namespace {
 using namespace df;
 constexpr int RUN = 4;  // outputs per thread along j3
 
-constexpr int DEPTH = 8;  // B rows in flight per warp
-
 __device__ __forceinline__ uint32_t s_addr(const void *p) {
   return (uint32_t)__cvta_generic_to_shared(p);
 }
 __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(s_addr(bar)), "r"(count)
                : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(s_addr(bar)),
-               "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t bytes,
-                                         uint64_t *bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::
-          "r"(s_addr(dst)),
-      "l"(src), "r"(bytes), "r"(s_addr(bar))
-      : "memory");
 }
 __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
   uint32_t ok;
@@ -101,29 +85,10 @@ __device__ __forceinline__ unsigned long long gtimer_ns() {
   asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
   return t;
 }
-// Wait for the phase with this parity, for at most limit_ns (0: every wait
-// runs out at once, without polling); a thread that timed out does not wait
-// again.
+// Wait for the phase with this parity, for at most limit_ns (not 0); a thread
+// that timed out does not wait again.
 __device__ __forceinline__ void mbar_wait(uint64_t *bar, uint32_t parity, bool &to,
                                           unsigned long long limit_ns) {
-  if (to) return;
-  if (limit_ns == 0) {
-    to = true;
-    return;
-  }
-  if (mbar_try_wait(bar, parity)) return;
-  const unsigned long long t0 = gtimer_ns();
-  while (!mbar_try_wait(bar, parity)) {
-    if (gtimer_ns() - t0 >= limit_ns) {
-      to = true;
-      return;
-    }
-  }
-}
-
-// mbar_wait for a nonzero limit
-__device__ __forceinline__ void mbar_wait_nz(uint64_t *bar, uint32_t parity, bool &to,
-                                             unsigned long long limit_ns) {
   if (to || mbar_try_wait(bar, parity)) return;
   const unsigned long long t0 = gtimer_ns();
   while (!mbar_try_wait(bar, parity)) {
@@ -222,32 +187,20 @@ __global__ void b2_pair_split_kernel(int N, const double *__restrict__ B, float2
   o[hp + 2] = (float)(v - (double)h);
 }
 
-// TMA: per-warp bulk-copy ring for B (requires contiguous, aligned warp
-// segments; see the launcher).  Otherwise __ldg one row ahead.
 // MAXT, MINB: CTA size bound and minimum resident CTAs per SM the register
 // allocation must allow (see kC64xShapes).  The kernel is bound by the latency
 // of its dependent double-float chains, so resident warps matter: chosen per
 // table by timing every shape (edb_qcalc_genB runs the comparison once).
-template <bool TMA, int MAXT, int MINB>
+template <int MAXT, int MINB>
 __global__ void __launch_bounds__(MAXT, MINB)
     calq64x_kernel(QParams p, int J2T, int LC, const float2 *__restrict__ B2,
-                   const float4 *__restrict__ fdf, double2 *__restrict__ partial,
-                   unsigned long long wait_ns) {
+                   const float4 *__restrict__ fdf, double2 *__restrict__ partial) {
   extern __shared__ __align__(128) unsigned char smem64[];
   const int N = p.N, P = p.P;
   const int R4 = (P + RUN - 1) / RUN;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int nwarps = (blockDim.x + 31) >> 5;
-  const int wthreads = min(32, (int)blockDim.x - warp * 32);  // threads in this warp
-  const unsigned wmask = wthreads == 32 ? 0xffffffffu : ((1u << wthreads) - 1u);
+  const int tid = threadIdx.x;
   const long long NN = (long long)N * N;
-  // shared memory: [nwarps][DEPTH] mbarriers, B rings [nwarps][DEPTH][32 threads x 4 pairs],
-  // then the f-hat plane [N][N]
-  uint64_t *bars = reinterpret_cast<uint64_t *>(smem64);
-  float2 *rings = reinterpret_cast<float2 *>(smem64 + 16 * ((nwarps * DEPTH * 8 + 15) / 16));
-  float4 *plane = reinterpret_cast<float4 *>(rings + (TMA ? (size_t)nwarps * DEPTH * 32 * RUN : 0));
-  uint64_t *mybar = bars + warp * DEPTH;
-  float2 *myring = rings + (size_t)warp * DEPTH * 32 * RUN;
+  float4 *plane = reinterpret_cast<float4 *>(smem64);  // the f-hat plane [N][N]
 
   const int r = tid % R4;
   const int j2l = tid / R4;
@@ -266,33 +219,6 @@ __global__ void __launch_bounds__(MAXT, MINB)
 #pragma unroll
   for (int a = 0; a < RUN; ++a) colc[a] = (j3_0 + a < P) ? a : 0;
 
-  // the warp's B segment: threads [32 warp, 32 warp + wthreads) are consecutive
-  // 4-pair runs, contiguous in the row (checked by the launcher)
-  const long long wcol = ((long long)j1 * P + (blockIdx.y * J2T + (warp * 32) / R4)) * P +
-                         ((warp * 32) % R4) * RUN;
-  const uint32_t seg_bytes = (uint32_t)(wthreads * RUN * sizeof(float2));
-  const int nrows = (c1 - c0) * N;  // rows this CTA streams
-  bool to = false;
-  int issued = 0;  // lane 0: rows its warp has issued into the ring
-  // the chunk's rows follow one another in the table
-  const float2 *rf_src = B2 + (long long)c0 * N * p.KC + wcol;  // next row to copy
-
-  if (TMA) {
-    if (lane == 0) {
-      for (int d = 0; d < DEPTH; ++d) mbar_init(&mybar[d], 1);
-      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncwarp(wmask);
-    if (lane == 0) {  // prologue: the first DEPTH rows
-      for (int q = 0; q < DEPTH && q < nrows; ++q) {
-        mbar_expect_tx(&mybar[q], seg_bytes);
-        bulk_g2s(myring + (size_t)q * 32 * RUN, rf_src, seg_bytes, &mybar[q]);
-        rf_src += p.KC;
-        ++issued;
-      }
-    }
-  }
-
   DF2 accA[RUN], accB[RUN];
 #pragma unroll
   for (int a = 0; a < RUN; ++a) {
@@ -303,7 +229,6 @@ __global__ void __launch_bounds__(MAXT, MINB)
   const int base3 = (j3_0 + p.sM) % N;  // m3 of output a = 0 at i3 = 0
   const int fi0 = p.sL % N;             // f_l entry at i3 = 0
   int cur_i1 = -1;
-  int q = 0;  // row counter within the chunk
   for (int line = c0; line < c1; ++line) {
     // line indices: i1, i2 (centred l); a1, a2 = (i + sL) mod N (f_l, FFTW
     // order); m2 = (j2 - i2 + sM) mod N.  Computed per line: counters kept
@@ -337,37 +262,14 @@ __global__ void __launch_bounds__(MAXT, MINB)
     int m3n = base3;  // value at i3 = 0
     int fi = fi0;
     float4 fl_next = __ldg(flrow + fi);
-    if (!TMA) {
 #pragma unroll
-      for (int a = 0; a < RUN; ++a) bcur[a] = __ldg(brow + colc[a]);
-    }
+    for (int a = 0; a < RUN; ++a) bcur[a] = __ldg(brow + colc[a]);
     for (int g = 0; g < N; g += RUN) {
 #pragma unroll
-      for (int t = 0; t < RUN; ++t, ++q) {
+      for (int t = 0; t < RUN; ++t) {
         const int i3 = g + t;
         if (i3 >= N) break;
-        if (TMA) {
-          const int slot = q % DEPTH;
-          mbar_wait(&mybar[slot], (uint32_t)((q / DEPTH) & 1), to, wait_ns);
-          const float4 *src = reinterpret_cast<const float4 *>(myring + ((size_t)slot * 32 + lane) * RUN);
-#pragma unroll
-          for (int h = 0; h < RUN / 2; ++h) {
-            const float4 v = src[h];
-            bcur[2 * h] = make_float2(v.x, v.y);
-            bcur[2 * h + 1] = make_float2(v.z, v.w);
-          }
-          // every lane has read the slot; refill it with row q + DEPTH unless a
-          // lane timed out (its copy may still be landing: the warp then
-          // issues nothing more, so at most one copy per slot is in flight)
-          const bool bad = __any_sync(wmask, to);
-          if (lane == 0 && !bad && q + DEPTH < nrows) {
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            mbar_expect_tx(&mybar[slot], seg_bytes);
-            bulk_g2s(myring + (size_t)slot * 32 * RUN, rf_src, seg_bytes, &mybar[slot]);
-            rf_src += p.KC;
-            ++issued;
-          }
-        } else if (i3 + 1 < N) {
+        if (i3 + 1 < N) {
           const float2 *bn = brow + (long long)(i3 + 1) * p.KC;
 #pragma unroll
           for (int a = 0; a < RUN; ++a) bnext[a] = __ldg(bn + colc[a]);
@@ -400,28 +302,9 @@ __global__ void __launch_bounds__(MAXT, MINB)
         for (int a = 0; a < RUN; ++a) df_axpy(accA[a], xr, nxr, nlr, nuh[a], ucs[a]);
 #pragma unroll
         for (int a = 0; a < RUN; ++a) df_axpy(accB[a], xi, nxi, nli, nuh[a], ucs[a]);
-        if (!TMA) {
 #pragma unroll
-          for (int a = 0; a < RUN; ++a) bcur[a] = bnext[a];
-        }
+        for (int a = 0; a < RUN; ++a) bcur[a] = bnext[a];
       }
-    }
-  }
-  if (TMA) {
-    if (__syncthreads_or(to)) {
-      if (lane == 0) {
-        atomicExch(&g_calq64x_status, 1);
-        // drain: row r went into slot r % DEPTH as its fill r / DEPTH, and a
-        // slot is refilled only after its previous copy landed, so only the
-        // last row issued into each slot can still be in flight
-        for (int sl = 0; sl < DEPTH && sl < issued; ++sl) {
-          const int last = sl + ((issued - 1 - sl) / DEPTH) * DEPTH;
-          bool t2 = false;
-          mbar_wait(&mybar[sl], (uint32_t)((last / DEPTH) & 1), t2, DRAIN_LIMIT_NS);
-        }
-      }
-      __syncwarp(wmask);
-      return;
     }
   }
   if (!ok) return;
@@ -660,7 +543,7 @@ __global__ void __launch_bounds__(MAXT, MINB)
 #pragma unroll
       for (int t = 0; t < RUN; ++t) {
         const int slot = ((q & 4) + t) / ROWS;
-        if (t % ROWS == 0) mbar_wait_nz(&mybar[slot], (uint32_t)((q >> 3) & 1), to, wait_ns);
+        if (t % ROWS == 0) mbar_wait(&mybar[slot], (uint32_t)((q >> 3) & 1), to, wait_ns);
         const float4 bv0 = ring_g[t * RS];
         const float4 bv1 = ring_g[t * RS + 1 - 2 * hsw];
         // every lane has read the slot's rows; refill it with the next ROWS
@@ -749,7 +632,6 @@ __global__ void __launch_bounds__(MAXT, MINB)
 
 struct C64xPlan {
   int J2T, tiles, threads, LC, nch;
-  bool tma;
   size_t smem;
 };
 
@@ -795,32 +677,26 @@ static C64pFn c64p_fn(int shape, int N) {
     default: return c64p_fn_s<4>(N);
   }
 }
-typedef void (*C64xFn)(QParams, int, int, const float2 *, const float4 *, double2 *,
-                       unsigned long long);
-template <bool TMA>
+typedef void (*C64xFn)(QParams, int, int, const float2 *, const float4 *, double2 *);
 static C64xFn c64x_fn(int shape) {
   switch (shape) {
-    case 0: return calq64x_kernel<TMA, kC64xShapes[0].maxt, kC64xShapes[0].minb>;
-    case 1: return calq64x_kernel<TMA, kC64xShapes[1].maxt, kC64xShapes[1].minb>;
-    case 2: return calq64x_kernel<TMA, kC64xShapes[2].maxt, kC64xShapes[2].minb>;
-    case 3: return calq64x_kernel<TMA, kC64xShapes[3].maxt, kC64xShapes[3].minb>;
-    default: return calq64x_kernel<TMA, kC64xShapes[4].maxt, kC64xShapes[4].minb>;
+    case 0: return calq64x_kernel<kC64xShapes[0].maxt, kC64xShapes[0].minb>;
+    case 1: return calq64x_kernel<kC64xShapes[1].maxt, kC64xShapes[1].minb>;
+    case 2: return calq64x_kernel<kC64xShapes[2].maxt, kC64xShapes[2].minb>;
+    case 3: return calq64x_kernel<kC64xShapes[3].maxt, kC64xShapes[3].minb>;
+    default: return calq64x_kernel<kC64xShapes[4].maxt, kC64xShapes[4].minb>;
   }
 }
 
-static size_t c64x_smem(int N, int threads, bool tma, bool op, int rows) {
+static size_t c64x_smem(int N, int threads, bool op, int rows) {
+  if (!op) return sizeof(float4) * (size_t)N * N;
   const int nwarps = (threads + 31) / 32;
-  if (op) {
-    return (size_t)nwarps * (PDEPTH / rows) * 8 +
-           2 * sizeof(float4) * (size_t)nwarps * PDEPTH * p64_box_threads(threads) +
-           2 * sizeof(float4) * (size_t)N * ((N + RUN - 1) / RUN * RUN);
-  }
-  size_t o = 16 * (size_t)((nwarps * DEPTH * 8 + 15) / 16);
-  if (tma) o += sizeof(float2) * (size_t)nwarps * DEPTH * 32 * RUN;
-  return o + sizeof(float4) * (size_t)N * N;
+  return (size_t)nwarps * (PDEPTH / rows) * 8 +
+         2 * sizeof(float4) * (size_t)nwarps * PDEPTH * p64_box_threads(threads) +
+         2 * sizeof(float4) * (size_t)N * ((N + RUN - 1) / RUN * RUN);
 }
 
-// Tile shape, TMA eligibility and the line-chunk count that makes the grid
+// Tile shape and the line-chunk count that makes the grid
 // whole waves of resident CTAs (cached per shape: the occupancy query is not
 // free).
 // l-lines of the longest plane list (all N^2 lines, or about half when paired)
@@ -831,19 +707,18 @@ static int c64x_lines(const QParams &p, bool paired) {
   return m * p.N;
 }
 
-static C64xPlan c64x_plan_compute(const QParams &p, bool aligned, int shape, bool paired);
-static C64xPlan c64x_plan(const QParams &p, bool aligned, int shape, bool paired) {
+static C64xPlan c64x_plan_compute(const QParams &p, int shape, bool paired);
+static C64xPlan c64x_plan(const QParams &p, int shape, bool paired) {
   static std::mutex mu;
   static std::map<long long, C64xPlan> cache;
   int dev = 0;
   cudaGetDevice(&dev);
   const long long key =
-      (((((long long)dev * 128 + p.N) * 4 + p.mode) * 2 + (aligned ? 1 : 0)) * 16 + shape) * 2 +
-      (paired ? 1 : 0);
+      ((((long long)dev * 128 + p.N) * 4 + p.mode) * 16 + shape) * 2 + (paired ? 1 : 0);
   std::lock_guard<std::mutex> lock(mu);
   auto it = cache.find(key);
   if (it != cache.end()) return it->second;
-  C64xPlan pl = c64x_plan_compute(p, aligned, shape, paired);
+  C64xPlan pl = c64x_plan_compute(p, shape, paired);
   cache[key] = pl;
   return pl;
 }
@@ -851,7 +726,7 @@ static C64xPlan c64x_plan(const QParams &p, bool aligned, int shape, bool paired
 // shape in [0, 2 kC64xNShapes): the kernel shape shape mod kC64xNShapes, with
 // the line chunks sized by whole waves (first half) or by the schedule model
 // (second half)
-static C64xPlan c64x_plan_compute(const QParams &p, bool aligned, int shape_in, bool paired) {
+static C64xPlan c64x_plan_compute(const QParams &p, int shape_in, bool paired) {
   C64xPlan pl;
   const int shape = shape_in % kC64xNShapes;
   const bool model = shape_in >= kC64xNShapes;
@@ -864,12 +739,9 @@ static C64xPlan c64x_plan_compute(const QParams &p, bool aligned, int shape_in, 
   pl.J2T = J2T;
   pl.tiles = tiles;
   pl.threads = J2T * R4;
-  pl.tma = op || (aligned && (p.P % RUN) == 0 && (p.P % J2T) == 0);
-  pl.smem = c64x_smem(p.N, pl.threads, pl.tma, op, kC64pShapes[shape].rows);
+  pl.smem = c64x_smem(p.N, pl.threads, op, kC64pShapes[shape].rows);
   int occ = 1;
-  const void *fn = op       ? (const void *)c64p_fn(shape, p.N)
-                   : pl.tma ? (const void *)c64x_fn<true>(shape)
-                            : (const void *)c64x_fn<false>(shape);
+  const void *fn = op ? (const void *)c64p_fn(shape, p.N) : (const void *)c64x_fn(shape);
   cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, pl.threads, pl.smem);
   if (occ < 1) occ = 1;
@@ -931,16 +803,11 @@ static C64xPlan c64x_plan_compute(const QParams &p, bool aligned, int shape_in, 
   return pl;
 }
 
-int calq64x_nchunk(const QParams &p, int *J2T_out) {
-  // upper bound over the variants, used to size the partial-sum buffer
+int calq64x_nchunk(const QParams &p, bool paired) {
+  // upper bound over the shapes, used to size the partial-sum buffer
   int n = 1;
   for (int shape = 0; shape < 2 * kC64xNShapes; ++shape)
-    for (int al = 0; al <= 1; ++al)
-      for (int pa = 0; pa <= 1; ++pa) {
-        const C64xPlan pl = c64x_plan(p, al != 0, shape, pa != 0);
-        if (J2T_out) *J2T_out = pl.J2T;
-        if (pl.nch > n) n = pl.nch;
-      }
+    n = std::max(n, c64x_plan(p, shape, paired).nch);
   return n;
 }
 
@@ -976,10 +843,9 @@ edb_status launch_calq64x(const QParams &p, const float2 *d_B2, const double2 *d
   if (shape < 0 || shape >= 2 * kC64xNShapes) shape = 0;
   if (paired && (p.P != p.N || (p.sM % p.N) != 0 || (p.sL % p.N) != p.N - p.n))
     return fail(EDB_EINVAL, "calq64x: pairs need the aliased index shifts");
-  const bool aligned = ((uintptr_t)d_B2 % 16) == 0;
-  if (paired && !aligned)
+  if (paired && ((uintptr_t)d_B2 % 16) != 0)
     return fail(EDB_EINVAL, "calq64x: the output-pair table must be 16-byte aligned");
-  const C64xPlan pl = c64x_plan(p, aligned, shape, paired);
+  const C64xPlan pl = c64x_plan(p, shape, paired);
   const dim3 grid((unsigned)p.P, (unsigned)pl.tiles, (unsigned)pl.nch);
   const int s = shape % kC64xNShapes;
   if (paired) {
@@ -998,8 +864,7 @@ edb_status launch_calq64x(const QParams &p, const float2 *d_B2, const double2 *d
   } else {
     fdf_split_kernel<<<(unsigned)((p.NQ + 255) / 256), 256, 0, st>>>(p.NQ, d_in, d_fdf);
     EDB_LAUNCHED();
-    (pl.tma ? c64x_fn<true>(s) : c64x_fn<false>(s))<<<grid, pl.threads, pl.smem, st>>>(
-        p, pl.J2T, pl.LC, d_B2, d_fdf, d_partial, wait_limit_ns());
+    c64x_fn(s)<<<grid, pl.threads, pl.smem, st>>>(p, pl.J2T, pl.LC, d_B2, d_fdf, d_partial);
     EDB_LAUNCHED();
   }
   return launch_calq64_reduce(p, pl.nch, d_partial, d_Q, st, paired);
