@@ -218,8 +218,8 @@ TcGeom tc_geom(int N);
 int tc_fours(int S, int N, int C, int sms);
 inline long long c32_table_floats(int N) {
   if (tc_takes(N)) {
-    const TcGeom g = tc_geom(N);
-    return (long long)N * c32_maxlist(N) * N * g.V * 128 * g.NC;
+    const int N4 = (N + 3) / 4 * 4;  // columns stored
+    return (long long)N * c32_maxlist(N) * N * tc_geom(N).V * 128 * N4;
   }
   const long long NQ = (long long)N * N * N;
   return (long long)N * c32_maxlist(N) * N * NQ;

@@ -311,6 +311,7 @@ TcGeom tc_geom(int N) {
 
 struct TcArgs {
   int N, S, CL, V, pitch, C, NST, FL;  // FL: steps per fold
+  int N4;                              // weight columns stored
   int first, end;                      // this launch's solves
   const float *B32;
   const float2 *fin;
@@ -337,7 +338,7 @@ struct TcCfg {
   // the largest form spills 76 bytes, at 200 the others' service threads do
   static constexpr int RC = NC == 32 && SG == 4 ? 200 : 192, RS = 256 - RC;
   static constexpr int NPB = NC == 32 ? 1 : 2;    // staged f_L planes
-  static constexpr int SB = 128 * NC * 4;         // bytes of a step's weights
+  static constexpr int SB = 128 * NC * 4;         // bytes of a ring stage
   static constexpr int PITCH = NC + 1;            // floats per lane of the fold's staging
   static_assert(NU >= 2, "tensor memory");
   static constexpr int oplen(int N) { return N - 1 + NCM; }  // rows of an operand array
@@ -445,6 +446,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) calqtc_kernel(const TcArgs a) {
     constexpr int CH = Cfg::CH, K = 2 * NC / CH;  // a tile comes in K reads
     constexpr int P1 = Cfg::PITCH;
     const uint32_t myB = ring + (uint32_t)(q * 32 + lane) * 16u;
+    const uint32_t lastB = (uint32_t)(a.N4 / 4 - 1) * 2048u;  // group NC / 4 - 1, or one less
     const uint32_t d0 = tm + ((uint32_t)(q * 32) << 16) + h * Cfg::DC;
     float *stage = reinterpret_cast<float *>(smem + o_stage) + h * 128 * P1;
     float4 *sums = reinterpret_cast<float4 *>(smem + o_sum);  // (hi, lo) of re and im
@@ -461,7 +463,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) calqtc_kernel(const TcArgs a) {
       for (int j = 0; j < NC / 4; ++j)
         asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];"
                      : "=l"(b[2 * j]), "=l"(b[2 * j + 1])
-                     : "r"(myB + (uint32_t)(stg * Cfg::SB + j * 2048)));
+                     : "r"(myB + (uint32_t)(stg * Cfg::SB) + (j == NC / 4 - 1 ? lastB : j * 2048u)));
     };
     // read k of this warpgroup's tile i of unit u
     auto read = [&](int u, int i, int k, uint32_t (&d)[CH]) {
@@ -698,14 +700,15 @@ __global__ void __launch_bounds__(TC_THREADS, 1) calqtc_kernel(const TcArgs a) {
     } else if (warp == 13) {
       // ------------------------------------------------------ weight stream
       const char *src = reinterpret_cast<const char *>(a.B32) +
-                        (long long)(k1 * c32_maxlist(N) + P0) * N * V * Cfg::SB;
+                        (long long)(k1 * c32_maxlist(N) + P0) * N * V * a.N4 * 512;
+      const uint32_t bytes = (uint32_t)a.N4 * 512u;  // of a step's weights
       int st = 0, sp = 1, n = 0;
       for (int i = 0; i < total; ++i) {
         mbar_doze(bar(BE + st), sp, lim, 100);
         // nothing more is issued once a wait ran out: the stage's last copy
         // may still be landing
         const bool on = lane == 0 && lim != 0;
-        bulk_load(ring + (uint32_t)(st * Cfg::SB), src + (long long)i * Cfg::SB, Cfg::SB,
+        bulk_load(ring + (uint32_t)(st * Cfg::SB), src + (long long)i * bytes, bytes,
                   bar(BF + st), on);
         n += on;
         if (++st == a.NST) {
@@ -912,6 +915,7 @@ edb_status launch_calqtc(int N, int S, const float *d_B32, const float2 *d_fin, 
   a.wait_ns = wait_limit_ns();
   EDB_TRY(calq32_status_ptr(&a.status));
   a.NST = 0;
+  a.N4 = (N + 3) / 4 * 4;
   const int four = tc_fours(S, N, C, device_sm_count());
 #define EDB_TC(NC)                                \
   EDB_TRY((launch_tc<NC, 4>(a, 0, four, st)));    \

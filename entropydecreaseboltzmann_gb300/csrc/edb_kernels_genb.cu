@@ -282,15 +282,19 @@ __global__ void genB_kernel(int N, int filter, double rval, const double *__rest
 
 // The pair table of the tensor-core batched kernel (tc_takes), the entries of
 // genB_kernel's in the order that kernel reads: one step's weights are 128 lanes
-// x NC columns, [k1][p][m2][v][j / 4][lane][j % 4].  Lane k2 CL + c, column j
-// of (k1, p, m2, v) weights the pair l = (l1 of p, k2 - m2, v CL + c),
-// m = (k1 - l1, m2, j - v CL), all mod N; places without a pair are zero.  One
+// x N4 columns (N and the zeros up to the next multiple of four),
+// [k1][p][m2][v][j / 4][lane][j % 4].  Lane k2 CL + c, column j of (k1, p, m2, v)
+// weights the pair l = (l1 of p, k2 - m2, v CL + c), m = (k1 - l1, m2, j - v CL),
+// all mod N; places without a pair are zero.  That is up to 1.9 times the pairs
+// (N = 13; 17 1.6, 31 1.1): with only the lanes in use stored, the kernel's addresses
+// cost it 5% (37 x N = 21 805 -> 851 us), and one copy per four columns 2 to 29%
+// (805 -> 886, 17 x N = 31 2.80 -> 3.61 ms).  One
 // thread writes the four columns of a 16-byte word.
 __global__ void genB32_tc_kernel(int N, int filter, double rval, const double *__restrict__ T,
                                  int amax, const double *__restrict__ sigma,
                                  const double *__restrict__ Bmm, TcGeom g, long long words,
                                  float4 *__restrict__ out) {
-  const int n = (N - 1) / 2, Q4 = g.NC / 4, ML = c32_maxlist(N);
+  const int n = (N - 1) / 2, Q4 = (N + 3) / 4, ML = c32_maxlist(N);
   const long long W = amax + 1;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < words;
        i += (long long)gridDim.x * blockDim.x) {
