@@ -346,6 +346,65 @@ struct TcCfg {
   static constexpr size_t stage() { return 2u * 128 * PITCH * 4; }
 };
 
+// One output (k1, k2, k3) over the planes [P0, P0 + np) of f (one solve), term by
+// term with the weight first, in calq32_kernel's form.  Products are formed
+// before they are weighted, and one that leaves FP32's range makes its output
+// infinite or no number; where the inputs are finite it is summed again here,
+// since its weighted terms may be in range.
+static __device__ float4 tc_direct(const TcArgs &a, const float2 *f, int k1, int k2, int k3, int P0,
+                                   int np) {
+  const int N = a.N, NN = N * N, plo = k1 / 2;
+  float4 h = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int p = P0; p < P0 + np; ++p) {
+    const int l1 = p <= plo ? p : k1 + 1 + (p - plo - 1), m1 = k1 < l1 ? k1 - l1 + N : k1 - l1;
+    for (int m2 = 0; m2 < N; ++m2) {
+      const int l2 = k2 < m2 ? k2 - m2 + N : k2 - m2;
+      const float2 *fl = f + l1 * NN + l2 * N, *fm = f + m1 * NN + m2 * N;
+      const float *line = a.B32 + ((long long)(k1 * c32_maxlist(N) + p) * N + m2) * a.V * a.N4 * 128;
+      float ax = 0.f, ay = 0.f, bx = 0.f, by = 0.f;  // sums of f_l.re and of f_l.im
+      for (int l3 = 0; l3 < N; ++l3) {
+        const int v = l3 / a.CL, c = l3 - v * a.CL, j = k3 < c ? k3 - c + N : k3 - c;
+        const float w = line[((long long)(v * (a.N4 / 4) + j / 4) * 128 + k2 * a.CL + c) * 4 + j % 4];
+        const float2 x = fl[l3], y = fm[k3 < l3 ? k3 - l3 + N : k3 - l3];
+        const float qx = w * y.x, qy = w * y.y;
+        ax = __fmaf_rn(x.x, qx, ax);
+        ay = __fmaf_rn(x.x, qy, ay);
+        bx = __fmaf_rn(x.y, qx, bx);
+        by = __fmaf_rn(x.y, qy, by);
+      }
+      two_sum(h.x, h.y, ax - by);
+      two_sum(h.z, h.w, ay + bx);
+    }
+  }
+  return h;
+}
+static __device__ __forceinline__ bool tc_finite(float4 h) {
+  return isfinite(h.x + h.y) && isfinite(h.z + h.w);
+}
+// The CTA's sums that are not finite though their solve's inputs are, again.
+// Everything is derived from the block's index anew, so that nothing is kept in
+// registers for this through the roles' loops.
+template <int SG>
+static __device__ __forceinline__ void tc_again(const TcArgs &a, float4 *sums) {
+  int block, tid;
+  asm volatile("mov.u32 %0, %%ctaid.x;\n mov.u32 %1, %%tid.x;" : "=r"(block), "=r"(tid));
+  const int N = a.N, NN = N * N, groups = (a.end - a.first + SG - 1) / SG, grp = block % groups;
+  const int chunk = block / groups % a.C, k1 = block / groups / a.C;
+  const int s0 = a.first + grp * SG, ns = min(SG, a.end - s0);
+  const int nlist = c32_nlist(N, k1), ppc = (nlist + a.C - 1) / a.C;
+  const int P0 = min(nlist, chunk * ppc), np = min(nlist, P0 + ppc) - P0;
+  for (int s = 0; s < ns; ++s) {
+    const float2 *f = a.fin + (long long)(s0 + s) * NN * N;
+    bool in = true;
+    for (int e = tid; e < NN * N; e += TC_THREADS) in &= isfinite(f[e].x) && isfinite(f[e].y);
+    if (__syncthreads_or(!in)) continue;
+    for (int e = tid; e < NN; e += TC_THREADS)
+      if (!tc_finite(sums[s * NN + e]))
+        sums[s * NN + e] = tc_direct(a, f, k1, e / N, e % N, P0, np);
+  }
+  __syncthreads();
+}
+
 // Barriers in the header (8 bytes each)
 enum {
   BF = 0,             // weights landed [MAX_STG]
@@ -815,6 +874,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1) calqtc_kernel(const TcArgs a) {
     }
   }
   __syncwarp();
+  // back to the launch's share each: what follows is all warps' code, and at a
+  // service thread's share it spills, which costs the loops above 2%
+  if (warp < 8)
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 128;");
+  else
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 128;");
   const bool aborted = __syncthreads_or(lim == 0) != 0;
   if (aborted) {
     if (tid == 0) {
@@ -825,7 +890,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) calqtc_kernel(const TcArgs a) {
         mbar_poll(bar(BF + i % a.NST), (uint32_t)((i / a.NST) & 1), DRAIN_LIMIT_NS);
     }
   } else {
-    const float4 *sums = reinterpret_cast<const float4 *>(smem + o_sum);
+    float4 *sums = reinterpret_cast<float4 *>(smem + o_sum);
+    bool odd = false;
+    for (int e = tid; e < ns * NN; e += TC_THREADS) odd |= !tc_finite(sums[e]);
+    if (__syncthreads_or(odd)) tc_again<SG>(a, sums);
     for (int e = tid; e < ns * NN; e += TC_THREADS) {
       const int s = e / NN, k23 = e - s * NN;
       const float4 h = sums[e];

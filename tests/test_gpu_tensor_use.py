@@ -36,7 +36,8 @@ def test_a_bad_solve_leaves_its_neighbours_bits_alone(edb, N, S, bad):
         q.calQ_batch_f32(S, f, out)
         others = [s for s in range(S) if s != at]
         assert torch.equal(out[others], good[others]), at
-        assert not torch.isfinite(torch.view_as_real(out[at])).all()
+        if not np.isfinite(bad):
+            assert not torch.isfinite(torch.view_as_real(out[at])).all()
     assert edb.device_status() == 0
 
 
