@@ -43,10 +43,14 @@
 // N = 13 5.9e-7 -> 5.1e-7 (6.6e-7), 21 8.5e-7 -> 7.0e-7 (8.3e-7).  The shorter sums
 // cost 1.5 to 6% (4096 of N = 13 9.20 -> 9.54 ms, 37 of N = 21 770 -> 806 us).
 //
-// What bounds it: the instruction issue of the hand-overs and of the A rows
-// beside the FMAs (a tile of N = 24 takes about 240 clocks an SM, its FMAs 60).
-// Measured, ms: 37 solves of N = 21 2.80 (calq32_kernel's plain-load path) ->
-// 0.80, 256 of N = 31 126 -> 31, 16 of N = 17 0.82 -> 0.16.
+// What bounds it: the hand-overs between the roles and the A rows beside the
+// FMAs (a tile of N = 21 takes about 256 clocks an SM, its FMAs 60; an SM with work
+// issues in 56% of its cycles, FMA pipe 17%, tensor pipe 12%).  Measured, ms, calq32_kernel's
+// plain-load path -> here: 37 solves of N = 21 2.80 -> 0.81, 256 of N = 31 126 -> 34,
+// 16 of N = 17 0.82 -> 0.16.
+//
+// Range: a solve with an infinity or a NaN is NaN throughout, as in calq32_kernel;
+// products that overflow before they are weighted see tc_direct.
 #include <algorithm>
 
 #include "edb_df.cuh"
