@@ -354,7 +354,8 @@ struct TcCfg {
 // term with the weight first, in calq32_kernel's form.  Products are formed
 // before they are weighted, and one that leaves FP32's range makes its output
 // infinite or no number; where the inputs are finite it is summed again here,
-// since its weighted terms may be in range.
+// since its weighted terms may be in range (37 of N = 21: 0.81 ms, 2.4 with one such
+// solve, 8.9 with all of them; a solve with a NaN costs nothing).
 static __device__ float4 tc_direct(const TcArgs &a, const float2 *f, int k1, int k2, int k3, int P0,
                                    int np) {
   const int N = a.N, NN = N * N, plo = k1 / 2;
